@@ -928,11 +928,15 @@ int launch_one_step(fn_ctx* c, bool do_drift, bool store_v) {
     return FN_OK;
 }
 
+/* Where a segment stands in its RunSimulationLoop call: inside it, at its end,
+   or before a last segment of a single step. */
+enum { SEG_INNER = 0, SEG_LAST = 1, SEG_BEFORE_ONE = 2 };
+
 /* One segment of a RunSimulationLoop call: the contact rebuild that opens
-   every grid_update_freq steps, then `len` steps; when `tail` the segment
-   ends the call, so its last step does not drift and the step before it
+   every grid_update_freq steps, then `len` steps.  The call's last step does
+   not drift, and the step before it, which may belong to the segment before,
    keeps the predicted velocity. */
-int launch_segment(fn_ctx* c, int len, bool tail) {
+int launch_segment(fn_ctx* c, int len, int place) {
     int r = do_rebuild(c);
     if (r) return r;
     for (int k = 0; k < len; ++k) {
@@ -940,24 +944,24 @@ int launch_segment(fn_ctx* c, int len, bool tail) {
             r = do_rebuild(c); /* gated: runs only when a bead moved too far */
             if (r) return r;
         }
-        const bool last = tail && k == len - 1;
-        r = launch_one_step(c, !last, tail && k == len - 2);
+        const bool last = place == SEG_LAST && k == len - 1;
+        r = launch_one_step(c, !last, (place == SEG_LAST && k == len - 2) || (place == SEG_BEFORE_ONE && k == len - 1));
         if (r) return r;
     }
     return FN_OK;
 }
 
 /* The segment through a CUDA graph captured on first use (kernel arguments
-   depend on the ping-pong parity, the length and whether it ends the call). */
-int run_segment(fn_ctx* c, int len, bool tail) {
-    if (!c->cfg.use_graphs || c->timing) return launch_segment(c, len, tail);
-    const auto key = std::make_tuple(c->cur, len, tail ? 1 : 0);
+   depend on the ping-pong parity, the length and its place in the call). */
+int run_segment(fn_ctx* c, int len, int place) {
+    if (!c->cfg.use_graphs || c->timing) return launch_segment(c, len, place);
+    const auto key = std::make_tuple(c->cur, len, place);
     auto it = c->graphs.find(key);
     if (it == c->graphs.end()) {
         const int cur0 = c->cur;
         const long long rb0 = c->rebuilds_done;
         CK(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
-        int r = launch_segment(c, len, tail);
+        int r = launch_segment(c, len, place);
         cudaGraph_t g = nullptr;
         const cudaError_t e = cudaStreamEndCapture(c->stream, &g);
         if (r) {
@@ -976,7 +980,7 @@ int run_segment(fn_ctx* c, int len, bool tail) {
     CK(cudaGraphLaunch(it->second, c->stream));
     c->graph_launches++;
     c->rebuilds_done++;
-    const int drifts = tail ? len - 1 : len;
+    const int drifts = place == SEG_LAST ? len - 1 : len;
     if (drifts & 1) c->cur = 1 - c->cur;
     return FN_OK;
 }
@@ -1804,7 +1808,8 @@ FN_API int fn_step(fn_ctx* c, int nsteps) {
        opened by a rebuild */
     for (int done = 0; done < nsteps;) {
         const int len = std::min(c->grid_update_freq, nsteps - done);
-        r = run_segment(c, len, done + len == nsteps);
+        const int left = nsteps - done - len;
+        r = run_segment(c, len, left == 0 ? SEG_LAST : left == 1 ? SEG_BEFORE_ONE : SEG_INNER);
         if (r) return r;
         done += len;
     }

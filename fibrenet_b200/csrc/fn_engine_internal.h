@@ -125,7 +125,7 @@ struct fn_ctx {
     long long device_bytes = 0;
     long long steps_done = 0, rebuilds_done = 0;
 
-    /* captured step segments: (parity, length, ends the call) -> graph */
+    /* captured step segments: (parity, length, place in the call) -> graph */
     std::map<std::tuple<int, int, int>, cudaGraphExec_t> graphs;
     long long graph_launches = 0;
 

@@ -16,6 +16,7 @@
 #include <cstdint>
 #include <cstdio>
 #include <cstring>
+#include <limits>
 #include <map>
 #include <mutex>
 #include <tuple>
@@ -313,6 +314,7 @@ int derive_net(fn_ctx* c, const fn_settings& s, FnNet& N, int net_index) {
 void pair_coeffs(int kind, const double* raw, FnPair& P) {
     std::memset(&P, 0, sizeof P);
     P.kind = kind;
+    P.lj_r2_min = std::numeric_limits<double>::infinity();
     if (kind == FN_PAIR_LJ) {
         P.c[0] = raw[0];
         P.c[1] = raw[1];
@@ -324,6 +326,13 @@ void pair_coeffs(int kind, const double* raw, FnPair& P) {
         double fr2 = sigma2 / r2;
         double fr6 = fr2 * fr2 * fr2;
         P.c[3] = 48.0 * epsilon * fr6 * (fr6 - 0.5) / r2;
+        P.lj_s2 = sigma2;
+        P.lj_e48 = 48.0 * epsilon;
+        /* sigma^2 / r^2 stays in [2^-80, 2^40], its sixth power and the
+           force far inside the normal range */
+        const double lo = std::ldexp(1.0, -40), hi = std::ldexp(1.0, 40), e = std::fabs(epsilon);
+        if (sigma2 >= lo && sigma2 <= hi && r2 <= hi && e >= std::ldexp(1.0, -100) && e <= std::ldexp(1.0, 100))
+            P.lj_r2_min = sigma2 * lo;
     } else if (kind == FN_PAIR_HS) {
         P.c[0] = raw[0];
     } else if (kind == FN_PAIR_HSR) {
@@ -843,6 +852,11 @@ fn::StepArgs step_args(fn_ctx* c, bool pingpong) {
     A.ch_flags = c->ch_flags.p;
     A.ch_status = c->ch_status.p;
     A.nb = (int)c->nb;
+    A.uniform = c->uniform ? 1 : 0;
+    if (c->uniform) {
+        A.net0 = c->nets_h[0];
+        A.pair0 = c->pairs_h[0];
+    }
     A.csr = c->csr.p;
     A.csr_region = c->csr_region;
     A.tile_items = c->tile_items.p;
@@ -1289,6 +1303,11 @@ static void set_totals(fn_ctx* c, long long nb, long long ns, long long na, long
     c->ns = ns;
     c->na = na;
     c->ncells = ncells;
+    /* one network whose bead types all meet by the same law: its constants
+       and that law travel as kernel parameters */
+    c->uniform = c->n_nets == 1 && !c->pairs_h.empty();
+    for (const FnPair& P : c->pairs_h)
+        if (std::memcmp(&P, &c->pairs_h[0], sizeof P) != 0) c->uniform = false;
     c->list_stride = (int)((nb + 31) / 32 * 32);
     c->grid_update_freq = c->info[0].grid_update_freq;
 }

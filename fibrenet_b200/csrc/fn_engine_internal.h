@@ -67,6 +67,7 @@ struct fn_ctx {
     std::vector<float4> sp_par_h;  // upload order (springs are not renumbered)
     std::vector<float2> an_par_h;
     bool damp = false;
+    bool uniform = false; /* one network, one pair law for all bead types */
     int grid_update_freq = 8;
 
     DevBuf<double4> pos[2], img[2];

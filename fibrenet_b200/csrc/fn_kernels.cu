@@ -29,6 +29,7 @@
 #include "fn_detmath.h"
 #include "fn_device.cuh"
 #include "fn_kernels.h"
+#include "fn_rounded.cuh"
 #include "fn_types.h"
 
 namespace fn {
@@ -60,14 +61,14 @@ __device__ __forceinline__ int spring_pts(double ax, double ay, double az, doubl
                                           double& fz, int& broke) {
     broke = 0;
     double dx = ax - bx, dy = ay - by, dz = az - bz;
-    double l = sqrt(dx * dx + dy * dy + dz * dz);
+    double l, il;
+    root_and_inverse(dx * dx + dy * dy + dz * dz, l, il);
     double factor = (double)par.x - l;
-    if (l != 0.0) l = 1.0 / l;
-    dx *= l;
-    dy *= l;
-    dz *= l;
+    dx *= il;
+    dy *= il;
+    dz *= il;
     if (type == 1) {
-        double stress = -(double)par.z * factor * l;
+        double stress = -(double)par.z * factor * il;
         if (fabs(stress) > (double)par.w) {
             broke = 1;
             return 0;
@@ -88,45 +89,71 @@ __device__ __forceinline__ int spring_alive_after(const StepArgs& A, int s) {
     return !broke;
 }
 
-/* Angle force (kernel.cl:291-348) from the image positions of b1 (t1),
-   b2 (t2), b3 (t3): pa acts on b1, pc on b3. */
+/* fn_acos with the root of its half-angle reduction from fn_rounded.cuh. */
+__device__ __forceinline__ double acos_rounded(double x) {
+    const double ax = fabs(x);
+    if (!(ax > 0.5)) return 1.5707963267948966 - fn_asin_poly(x); /* NaN stays NaN */
+    const double h = (1.0 - ax) * 0.5;
+    double s;
+    if (fn_fast_range(h))
+        s = root_from(h, rsqrt_seeded(h));
+    else
+        s = sqrt(h);
+    const double a = 2.0 * fn_asin_poly(s);
+    return x > 0.0 ? a : 3.141592653589793 - a;
+}
+
+/* Angle force (kernel.cl:291-348) from the arms ba = b1 - b2 and cb = b2 - b3,
+   their lengths and the inverses of those (correctly rounded): pa acts on b1,
+   pc on b3.  Swapping the arms swaps pa and pc bit for bit. */
+__device__ __forceinline__ void angle_arms(double bax, double bay, double baz, double cbx, double cby, double cbz,
+                                           double l_ba, double il_ba, double l_bc, double il_bc, float2 par,
+                                           double& pax, double& pay, double& paz, double& pcx, double& pcy,
+                                           double& pcz) {
+    const double bcx = -cbx, bcy = -cby, bcz = -cbz;
+    const double dot = bax * bcx + bay * bcy + baz * bcz;
+    const double ll = l_ba * l_bc;
+    const bool fast = fn_fast_range(ll);
+    double dotp = fast ? quotient(dot, ll, recip_from(ll, il_ba * il_bc)) : dot / ll;
+    if (dotp < -1.0) dotp = -0.999999;
+    if (dotp > 1.0) dotp = 0.999999;
+    const double angle = acos_rounded(dotp);
+    const double magnitude = -2.0 * (double)par.y * (angle - (double)par.x);
+    const double fa = fast ? quotient(magnitude, l_ba, il_ba) : magnitude / l_ba;
+    const double fc = fast ? quotient(magnitude, l_bc, il_bc) : magnitude / l_bc;
+    const double tx = bay * bcz - baz * bcy;
+    const double ty = baz * bcx - bax * bcz;
+    const double tz = bax * bcy - bay * bcx;
+    double ln, il;
+    pax = (bay * tz - baz * ty);
+    pay = (baz * tx - bax * tz);
+    paz = (bax * ty - bay * tx);
+    root_and_inverse(pax * pax + pay * pay + paz * paz, ln, il);
+    il *= fa;
+    pax *= il;
+    pay *= il;
+    paz *= il;
+    pcx = (cby * tz - cbz * ty);
+    pcy = (cbz * tx - cbx * tz);
+    pcz = (cbx * ty - cby * tx);
+    root_and_inverse(pcx * pcx + pcy * pcy + pcz * pcz, ln, il);
+    il *= fc;
+    pcx *= il;
+    pcy *= il;
+    pcz *= il;
+}
+
+/* The same from the image positions of b1 (t1), b2 (t2), b3 (t3). */
 __device__ __forceinline__ void angle_pts(double t1x, double t1y, double t1z, double t2x,
                                           double t2y, double t2z, double t3x, double t3y,
                                           double t3z, float2 par, double& pax, double& pay,
                                           double& paz, double& pcx, double& pcy, double& pcz) {
     const double bax = t1x - t2x, bay = t1y - t2y, baz = t1z - t2z;
-    const double bcx = t3x - t2x, bcy = t3y - t2y, bcz = t3z - t2z;
-    const double cbx = bcx * -1.0, cby = bcy * -1.0, cbz = bcz * -1.0;
-    const double l_ba = sqrt(bax * bax + bay * bay + baz * baz);
-    const double l_bc = sqrt(bcx * bcx + bcy * bcy + bcz * bcz);
-    double dotp = (bax * bcx + bay * bcy + baz * bcz) / (l_ba * l_bc);
-    if (dotp < -1.0) dotp = -0.999999;
-    if (dotp > 1.0) dotp = 0.999999;
-    const double angle = fn_acos(dotp);
-    const double magnitude = -2.0 * (double)par.y * (angle - (double)par.x);
-    const double fa = magnitude / l_ba;
-    const double fc = magnitude / l_bc;
-    const double tx = bay * bcz - baz * bcy;
-    const double ty = baz * bcx - bax * bcz;
-    const double tz = bax * bcy - bay * bcx;
-    pax = (bay * tz - baz * ty);
-    pay = (baz * tx - bax * tz);
-    paz = (bax * ty - bay * tx);
-    double ln = sqrt(pax * pax + pay * pay + paz * paz);
-    if (ln != 0.0) ln = 1.0 / ln;
-    ln *= fa;
-    pax *= ln;
-    pay *= ln;
-    paz *= ln;
-    pcx = (cby * tz - cbz * ty);
-    pcy = (cbz * tx - cbx * tz);
-    pcz = (cbx * ty - cby * tx);
-    ln = sqrt(pcx * pcx + pcy * pcy + pcz * pcz);
-    if (ln != 0.0) ln = 1.0 / ln;
-    ln *= fc;
-    pcx *= ln;
-    pcy *= ln;
-    pcz *= ln;
+    const double cbx = t2x - t3x, cby = t2y - t3y, cbz = t2z - t3z;
+    double la, ila, lc, ilc;
+    root_and_inverse(bax * bax + bay * bay + baz * baz, la, ila);
+    root_and_inverse(cbx * cbx + cby * cby + cbz * cbz, lc, ilc);
+    angle_arms(bax, bay, baz, cbx, cby, cbz, la, ila, lc, ilc, par, pax, pay, paz, pcx, pcy, pcz);
 }
 
 __device__ __forceinline__ void angle_eval(const StepArgs& A, int4 b, float2 par, double& pax,
@@ -139,57 +166,55 @@ __device__ __forceinline__ void angle_eval(const StepArgs& A, int4 b, float2 par
               pcz);
 }
 
-/* One contact-list entry (kernel.cl:835-999): force on bead i. */
-__device__ __forceinline__ int contact_eval(const FnNet& N, const FnPair* __restrict__ pairs,
-                                            double4 pi, double4 pj, double& Rx, double& Ry,
-                                            double& Rz) {
+/* One contact-list entry (kernel.cl:835-999) under the pair law P: force on
+   bead i.  Roots, reciprocals and quotients of the distance share one seed
+   (fn_rounded.cuh); distances outside its range take the operators. */
+__device__ __forceinline__ int contact_force(const FnNet& N, const FnPair& law, double4 pi, double4 pj, double& Rx,
+                                             double& Ry, double& Rz) {
+    const FnPair* P = &law;
     double rx = pi.x - pj.x, ry = pi.y - pj.y, rz = pi.z - pj.z;
     double length = rx * rx + ry * ry + rz * rz;
     length = min_image(N, rx, ry, rz, length, N.force_mi);
-    const int pid = N.pair_base + getadress(w_type(pi.w), w_type(pj.w), N.types_num);
-    const FnPair* P = pairs + pid;
     const int kind = P->kind;
     if (kind == 1) {
-        if (length < N.cutoff_sq) {
-            const double r2 = length;
+        if (!(length < N.cutoff_sq)) return 0;
+        const double r2 = length;
+        double fpr;
+        if (r2 >= P->lj_r2_min) {
+            const double y = rsqrt_seeded(r2);
+            const double r = root_from(r2, y);
+            if (!(r < P->c[2])) return 0;
+            length = recip_from(r, y);
+            const double ir2 = recip_from(r2, y * y);
+            const double fr2 = quotient(P->lj_s2, r2, ir2);
+            const double fr6 = fr2 * fr2 * fr2;
+            fpr = quotient(P->lj_e48 * fr6 * (fr6 - 0.5), r2, ir2);
+        } else {
             length = sqrt(length);
-            if (length < P->c[2]) {
-                double sigma2 = P->c[0];
-                const double epsilon = P->c[1];
-                sigma2 *= sigma2;
-                const double fr2 = sigma2 / r2;
-                const double fr6 = fr2 * fr2 * fr2;
-                double fpr = 48.0 * epsilon * fr6 * (fr6 - 0.5) / r2;
-                fpr -= P->c[3];
-                length = (length != 0.0) ? 1.0 / length : 0.0;
-                Rx = fpr * (rx * length);
-                Ry = fpr * (ry * length);
-                Rz = fpr * (rz * length);
-                return 1;
-            }
-        }
-        return 0;
-    }
-    if (kind == 2) {
-        length = sqrt(length);
-        const double K = P->c[0];
-        double penetration = ((double)w_radius(pi.w) + (double)w_radius(pj.w)) - length;
-        if (penetration > 0.0) {
+            if (!(length < P->c[2])) return 0;
+            const double fr2 = P->lj_s2 / r2;
+            const double fr6 = fr2 * fr2 * fr2;
+            fpr = P->lj_e48 * fr6 * (fr6 - 0.5) / r2;
             length = (length != 0.0) ? 1.0 / length : 0.0;
-            penetration *= K;
-            Rx = penetration * (rx * length);
-            Ry = penetration * (ry * length);
-            Rz = penetration * (rz * length);
-            return 1;
         }
-        return 0;
+        fpr -= P->c[3];
+        Rx = fpr * (rx * length);
+        Ry = fpr * (ry * length);
+        Rz = fpr * (rz * length);
+        return 1;
     }
-    if (kind == 4) {
+    double mag, inv;
+    if (kind == 2) {
+        root_and_inverse(length, length, inv);
+        mag = ((double)w_radius(pi.w) + (double)w_radius(pj.w)) - length;
+        if (!(mag > 0.0)) return 0;
+        mag *= P->c[0];
+    } else if (kind == 4) {
         /* extension, no counterpart in the reference: penalty spring K (c1)
            on the overlap plus a soft harmonic repulsion k (c2) below rc (c3) */
-        length = sqrt(length);
+        root_and_inverse(length, length, inv);
         const double penetration = ((double)w_radius(pi.w) + (double)w_radius(pj.w)) - length;
-        double mag = 0.0;
+        mag = 0.0;
         int acts = 0;
         if (penetration > 0.0) {
             mag += penetration * P->c[0];
@@ -199,29 +224,28 @@ __device__ __forceinline__ int contact_eval(const FnNet& N, const FnPair* __rest
             mag += (P->c[2] - length) * P->c[1];
             acts = 1;
         }
-        if (acts) {
-            length = (length != 0.0) ? 1.0 / length : 0.0;
-            Rx = mag * (rx * length);
-            Ry = mag * (ry * length);
-            Rz = mag * (rz * length);
-        }
-        return acts;
-    }
-    if (kind == 3) {
-        if (length < P->c[3]) {
-            length = sqrt(length);
-            double factor = (P->c[1] - length);
-            factor *= P->c[0]; /* both arms of kernel.cl:970-973 multiply by K */
-            factor += (P->c[5] - length) * P->c[4];
-            length = (length != 0.0) ? 1.0 / length : 0.0;
-            Rx = factor * (rx * length);
-            Ry = factor * (ry * length);
-            Rz = factor * (rz * length);
-            return 1;
-        }
+        if (!acts) return 0;
+    } else if (kind == 3) {
+        if (!(length < P->c[3])) return 0;
+        root_and_inverse(length, length, inv);
+        mag = (P->c[1] - length);
+        mag *= P->c[0]; /* both arms of kernel.cl:970-973 multiply by K */
+        mag += (P->c[5] - length) * P->c[4];
+    } else {
         return 0;
     }
-    return 0;
+    Rx = mag * (rx * inv);
+    Ry = mag * (ry * inv);
+    Rz = mag * (rz * inv);
+    return 1;
+}
+
+/* The same with the law looked up by the beads' types. */
+__device__ __forceinline__ int contact_eval(const FnNet& N, const FnPair* __restrict__ pairs,
+                                            double4 pi, double4 pj, double& Rx, double& Ry,
+                                            double& Rz) {
+    return contact_force(N, pairs[N.pair_base + getadress(w_type(pi.w), w_type(pj.w), N.types_num)], pi, pj, Rx, Ry,
+                         Rz);
 }
 
 /* AdvancePosition (kernel.cl:200-250) on registers: returns the drifted
@@ -291,46 +315,29 @@ __device__ __forceinline__ void base_force(const StepArgs& A, const FnNet& N, in
     }
 }
 
-/* Contacts, AdvanceVelocity and the next step's AdvancePosition for bead i,
-   given its base + bonded force (Fx, Fy, Fz) in FP64. */
-template <bool DAMP, bool DRIFT, bool STORE_V>
-__device__ __forceinline__ void kick_drift_store(const StepArgs& A, const FnNet& N, int i,
-                                                 double4 p, double Fx, double Fy, double Fz);
-
-template <bool DAMP, bool DRIFT, bool STORE_V>
-__device__ __forceinline__ void finish_bead(const StepArgs& A, const FnNet& N, int i, double4 p,
-                                            double Fx, double Fy, double Fz) {
-    /* contacts */
-    int n = A.list_count[i];
-    if (n > A.list_cap) n = A.list_cap;
-    const int* __restrict__ lst = A.list + i;
-    for (int k = 0; k < n; ++k) {
-        const int j = lst[(size_t)k * A.list_stride];
-        double Rx, Ry, Rz;
-        if (contact_eval(N, A.pairs, p, A.pos_in[j], Rx, Ry, Rz)) {
-            Fx += Rx;
-            Fy += Ry;
-            Fz += Rz;
-        }
-    }
-    kick_drift_store<DAMP, DRIFT, STORE_V>(A, N, i, p, Fx, Fy, Fz);
-}
+/* Flags of the step kernels: what a step does after the kick, and the terms
+   that the chain kernel's forces-only form evaluates. */
+enum { FN_STEP_SPRINGS = 1, FN_STEP_ANGLES = 2, FN_STEP_CONTACTS = 4, FN_STEP_DRIFT = 8, FN_STEP_STORE_V = 16 };
 
 /* AdvanceVelocity and the next AdvancePosition for bead i with its complete
    force (Fx, Fy, Fz), then the stores. */
-template <bool DAMP, bool DRIFT, bool STORE_V>
-__device__ __forceinline__ void kick_drift_store(const StepArgs& A, const FnNet& N, int i,
-                                                 double4 p, double Fx, double Fy, double Fz) {
+template <bool DAMP>
+__device__ __forceinline__ void kick_drift(const StepArgs& A, const FnNet& N, int i, double4 p, double Fx, double Fy,
+                                           double Fz, bool do_drift, bool store_v) {
+    /* loaded before the finiteness test: behind its branch these loads, and
+       with them every load of the kernel that reaches DRAM, take twice as
+       long (1M-bead tensile step 204 us against 108, the same sectors, hits
+       and DRAM bytes; networks that fit L2 see no difference) */
+    double4 im = A.img_in[i];
+    const float4 fo = A.force[i];
+    const float4 vo = A.vold[i];
     const float fx = (float)Fx, fy = (float)Fy, fz = (float)Fz;
     if (!(isfinite(fx) && isfinite(fy) && isfinite(fz)))
         atomicAdd(A.counters + FN_CNT_NONFINITE, 1ull);
 
     /* AdvanceVelocity, kernel.cl:451-462 */
-    double4 im = A.img_in[i];
     const double minv = im.w;
     const double half_dt = N.half_dt * minv;
-    const float4 fo = A.force[i];
-    const float4 vo = A.vold[i];
     double tx = (double)fx, ty = (double)fy, tz = (double)fz;
     tx += (double)fo.x;
     ty += (double)fo.y;
@@ -341,17 +348,42 @@ __device__ __forceinline__ void kick_drift_store(const StepArgs& A, const FnNet&
     A.force[i] = make_float4(fx, fy, fz, 0.0f);
     A.vold[i] = make_float4(vox, voy, voz, 0.0f);
 
-    if (DRIFT) {
+    if (do_drift) {
         float4 v;
         drift(N, minv, fx, fy, fz, vox, voy, voz, p, im, v);
         A.pos_out[i] = p;
         A.img_out[i] = im;
-        if (DAMP || STORE_V) A.vel[i] = v;
+        if (store_v) A.vel[i] = v;
     }
 }
 
-template <bool DAMP, bool DRIFT, bool STORE_V>
-__global__ void __launch_bounds__(512) k_step(const StepArgs A) {
+/* Contacts, AdvanceVelocity and the next step's AdvancePosition for bead i,
+   given its base + bonded force (Fx, Fy, Fz) in FP64.  The next list index is
+   loaded one item ahead. */
+template <bool DAMP, bool UNIFORM>
+__device__ __forceinline__ void finish_bead(const StepArgs& A, const FnNet& N, int i, double4 p, double Fx, double Fy,
+                                            double Fz, int flags) {
+    int n = A.list_count[i];
+    if (n > A.list_cap) n = A.list_cap;
+    const int* row = A.list + i;
+    int jn = *row;
+    for (int k = 0; k < n; ++k) {
+        const int j = jn;
+        if (k + 1 < A.list_cap) row += A.list_stride;
+        jn = *row;
+        double Rx, Ry, Rz;
+        if (UNIFORM ? contact_force(N, A.pair0, p, A.pos_in[j], Rx, Ry, Rz)
+                    : contact_eval(N, A.pairs, p, A.pos_in[j], Rx, Ry, Rz)) {
+            Fx += Rx;
+            Fy += Ry;
+            Fz += Rz;
+        }
+    }
+    kick_drift<DAMP>(A, N, i, p, Fx, Fy, Fz, (flags & FN_STEP_DRIFT) != 0, DAMP || (flags & FN_STEP_STORE_V));
+}
+
+template <bool DAMP>
+__global__ void __launch_bounds__(512) k_step(const __grid_constant__ StepArgs A, int flags) {
     const FnTile t = A.tiles[blockIdx.x];
     const int i = t.begin + (int)threadIdx.x;
     if (i >= t.end) return;
@@ -414,7 +446,7 @@ __global__ void __launch_bounds__(512) k_step(const StepArgs A) {
         }
     }
 
-    finish_bead<DAMP, DRIFT, STORE_V>(A, N, i, p, Fx, Fy, Fz);
+    finish_bead<DAMP, false>(A, N, i, p, Fx, Fy, Fz, flags);
 }
 
 /* The same step with the bonded terms evaluated once per tile: the block
@@ -422,8 +454,8 @@ __global__ void __launch_bounds__(512) k_step(const StepArgs A) {
    shared memory (flag bits: 1 force acts, 2 broke this step, 4 alive at step
    start), then each thread gathers its bead's terms from the shared slots in
    the same order as k_step, so the result is bit-identical to k_step. */
-template <bool DAMP, bool DRIFT, bool STORE_V>
-__global__ void __launch_bounds__(512) k_step_tiled(const StepArgs A) {
+template <bool DAMP, bool UNIFORM>
+__global__ void __launch_bounds__(512) k_step_tiled(const __grid_constant__ StepArgs A, int flags) {
     extern __shared__ double smem[];
     const int t = blockIdx.x;
     const FnTile tile = A.tiles[t];
@@ -471,7 +503,7 @@ __global__ void __launch_bounds__(512) k_step_tiled(const StepArgs A) {
 
     const int i = tile.begin + (int)threadIdx.x;
     if (i >= tile.end) return;
-    const FnNet& N = A.nets[tile.net];
+    const FnNet& N = UNIFORM ? A.net0 : A.nets[tile.net];
     const double4 p = A.pos_in[i];
     double Fx, Fy, Fz;
     base_force<DAMP>(A, N, i, p, Fx, Fy, Fz);
@@ -513,7 +545,7 @@ __global__ void __launch_bounds__(512) k_step_tiled(const StepArgs A) {
             Fz += -o[2] - o[5];
         }
     }
-    finish_bead<DAMP, DRIFT, STORE_V>(A, N, i, p, Fx, Fy, Fz);
+    finish_bead<DAMP, UNIFORM>(A, N, i, p, Fx, Fy, Fz, flags);
 }
 
 /* Exclusive prefix sum of v over the block (any size up to 1024); total
@@ -549,163 +581,143 @@ __device__ __forceinline__ int block_scan_any(int v, int* warp_sums, int& total)
 
 /* Step kernel for networks in chain form (every spring joins consecutive
    beads j, j+1 and every angle is centred on its middle bead, as fibres
-   are).  The block stages the image positions of its beads plus two halo
-   beads on each side in shared memory, evaluates every spring and angle
-   touching its beads once (springs first: an HR_FL angle dies with either of
-   its springs in the same step, kernel.cl:274-286), then each thread adds its
-   bead's terms in ascending bond order -- previous spring, next spring,
-   angles centred on j-1, j, j+1 -- which is the order of the incidence path,
-   so both produce identical bits.  Statuses are written back by the owning
-   thread.  FORCES_ONLY evaluates the selected terms alone (no base force, no
-   kick or drift, no status change). */
-template <bool DAMP, bool DRIFT, bool STORE_V, bool FORCES_ONLY>
-/* At most 256 threads per block and 4 such blocks per SM, i.e. at most 64
-   registers: the kernel waits on dependent loads of contact partners, and
-   both resident warps and the registers that keep the next list index in
-   flight hide that latency (measured on the 1M-bead tensile network: 0.135 ms
-   per step at 64 registers, 0.144 ms at 48 registers, 0.154 ms at 76). */
-__global__ void __launch_bounds__(kChainMaxBlock, 4) k_step_chain(const StepArgs A, int terms) {
+   are).  Thread t of a block works for bead j = tile begin - 2 + t (the tile
+   and a two-bead halo on each side): the block puts the image positions in
+   shared memory, then each thread evaluates the spring (j, j+1) and the
+   angle centred on j (springs first: an HR_FL angle dies with either of its
+   springs in the same step, kernel.cl:274-286), and the tile's threads add
+   their bead's terms in ascending bond order -- previous spring, next
+   spring, angles centred on j-1, j, j+1 -- which is the order of the
+   incidence path, so both produce identical bits.  A spring listed from its
+   upper bead and an angle listed from its far arm give the same bits as the
+   forward ones (every operation is symmetric under the swap), so the
+   records' direction is not read.  An angle takes its arms' lengths and
+   their inverses from the springs' threads.  FORCES_ONLY evaluates the
+   selected terms alone (no base force, no kick or drift, no status change).
+   UNIFORM reads the network's constants and its one pair law from the kernel
+   parameters, i.e. as constant operands, instead of loading them for every
+   contact (1M-bead tensile step 108 us against 120 with them loaded); contexts
+   with several networks or laws take the other form.
+   Bound by instruction issue and the latency of dependent loads and FP64
+   chains, not by DRAM (229 MB per 1M-bead step).  Sharing the roots' seeds
+   and the arms' lengths took it from 71.7M to 56.5M warp instructions: 130 to
+   108 us on the 1M-bead tensile network, 600 to 526 us on the 4M-bead mat, 24
+   to 20 us at 111k beads (one wave of blocks).  At most 256 threads per block
+   and 4 such blocks per SM, i.e. 64 registers: both resident warps and the
+   registers that keep the next list index in flight hide the loads' latency. */
+template <bool DAMP, bool FORCES_ONLY, bool UNIFORM>
+__global__ void __launch_bounds__(kChainMaxBlock, 4) k_step_chain(const __grid_constant__ StepArgs A, int flags) {
     extern __shared__ __align__(32) unsigned char smem_raw[];
     const FnTile tile = A.tiles[blockIdx.x];
-    const int b0 = tile.begin, n = tile.end - tile.begin;
+    const int tid = threadIdx.x, n = tile.end - tile.begin;
+    const int i = tile.begin - 2 + tid; /* this thread's bead */
     const ChainSmem L = chain_smem_layout(blockDim.x);
-    double* s_img = reinterpret_cast<double*>(smem_raw + L.img);  /* slot u <-> bead b0 - 2 + u */
-    double* s_spf = reinterpret_cast<double*>(smem_raw + L.spf);  /* lower bead b0 - 2 + u */
-    double* s_ang = reinterpret_cast<double*>(smem_raw + L.ang);  /* centre bead b0 - 1 + u */
-    unsigned char* s_flag = smem_raw + L.flag;
-    unsigned char* s_stat = smem_raw + L.stat;
-    unsigned char* s_tsp = smem_raw + L.tsp; /* spring term: 1 acts, 2 broke, 4 alive at start */
-    unsigned char* s_tan = smem_raw + L.tan; /* angle term alive */
-    const int tid = threadIdx.x;
+    double* s_img = reinterpret_cast<double*>(smem_raw + L.img);
+    double2* s_len = reinterpret_cast<double2*>(smem_raw + L.len);
+    double* s_spf = reinterpret_cast<double*>(smem_raw + L.spf);
+    double* s_ang = reinterpret_cast<double*>(smem_raw + L.ang);
+    unsigned char* s_ok = smem_raw + L.ok;
 
-    for (int u = tid; u < n + 4; u += blockDim.x) {
-        const int j = b0 - 2 + u;
-        unsigned char fl = 0, st = 0;
-        if (j >= 0 && j < A.nb) {
-            const double4 q = A.img_in[j];
-            s_img[3 * u] = q.x;
-            s_img[3 * u + 1] = q.y;
-            s_img[3 * u + 2] = q.z;
-            fl = A.ch_flags[j];
-            st = A.ch_status[j];
-        }
-        s_flag[u] = fl;
-        s_stat[u] = st;
+    unsigned fl = 0, st0 = 0;
+    double x = 0.0, y = 0.0, z = 0.0;
+    if (tid < n + 4 && i >= 0 && i < A.nb) {
+        const double4 q = A.img_in[i];
+        x = q.x;
+        y = q.y;
+        z = q.z;
+        fl = A.ch_flags[i];
+        st0 = A.ch_status[i];
     }
+    s_img[3 * tid] = x;
+    s_img[3 * tid + 1] = y;
+    s_img[3 * tid + 2] = z;
     __syncthreads();
 
-    const bool want_sp = !FORCES_ONLY || (terms & 1);
-    const bool want_an = !FORCES_ONLY || (terms & 2);
-    for (int u = tid; u < n + 3; u += blockDim.x) {
-        const unsigned fl = s_flag[u];
-        unsigned char tf = 0;
-        if (fl & FN_CH_SPRING) {
-            const int alive0 = s_stat[u] & 1;
-            tf = (unsigned char)(alive0 << 2);
-            if (alive0 && !(fl & FN_CH_SP_INERT)) {
-                const int j = b0 - 2 + u;
-                const float4 par = A.ch_sp[j];
-                const double* a = s_img + 3 * ((fl & FN_CH_SP_REV) ? u + 1 : u);
-                const double* b = s_img + 3 * ((fl & FN_CH_SP_REV) ? u : u + 1);
-                double fx = 0.0, fy = 0.0, fz = 0.0;
-                int broke;
-                const int acts = spring_pts(a[0], a[1], a[2], b[0], b[1], b[2], par,
-                                            (fl & FN_CH_SP_FL) ? 1 : 0, fx, fy, fz, broke);
-                s_spf[3 * u] = fx;
-                s_spf[3 * u + 1] = fy;
-                s_spf[3 * u + 2] = fz;
-                tf |= (unsigned char)(acts | (broke << 1));
+    /* spring (i, i+1): force on bead i (kernel.cl:377-424) */
+    double l = 0.0, il = 0.0;
+    double gx = 0.0, gy = 0.0, gz = 0.0;
+    unsigned st = st0; /* statuses after this step */
+    if (tid < n + 3) {
+        x -= s_img[3 * tid + 3];
+        y -= s_img[3 * tid + 4];
+        z -= s_img[3 * tid + 5];
+        root_and_inverse(x * x + y * y + z * z, l, il);
+        if ((fl & FN_CH_SPRING) && (st0 & 1) && !(fl & FN_CH_SP_INERT)) {
+            const float4 par = A.ch_sp[i];
+            double factor = (double)par.x - l;
+            if ((fl & FN_CH_SP_FL) && fabs(-(double)par.z * factor * il) > (double)par.w) {
+                st &= ~1u; /* breaks: no force from this step on (kernel.cl:391-397) */
+            } else if (!FORCES_ONLY || (flags & FN_STEP_SPRINGS)) {
+                factor *= (double)par.y;
+                gx = x * il * factor;
+                gy = y * il * factor;
+                gz = z * il * factor;
             }
         }
-        s_tsp[u] = tf;
+        s_len[tid] = make_double2(l, il);
+        s_spf[3 * tid] = gx;
+        s_spf[3 * tid + 1] = gy;
+        s_spf[3 * tid + 2] = gz;
+        s_ok[tid] = (unsigned char)((fl & FN_CH_SPRING) && (st & 1));
     }
     __syncthreads();
 
-    for (int u = tid; u < n + 2; u += blockDim.x) {
-        const unsigned fl = s_flag[u + 1];
-        int alive = (fl & FN_CH_ANGLE) && (s_stat[u + 1] & 2);
-        if (alive && (fl & FN_CH_AN_FL)) {
-            const unsigned f1 = s_tsp[u], f2 = s_tsp[u + 1];
-            if (!((f1 & 4) && !(f1 & 2)) || !((f2 & 4) && !(f2 & 2))) alive = 0;
+    /* angle centred on bead i */
+    double cx = 0.0, cy = 0.0, cz = 0.0; /* its force on bead i */
+    if (tid >= 1 && tid < n + 3) {
+        double pax = 0.0, pay = 0.0, paz = 0.0, pcx = 0.0, pcy = 0.0, pcz = 0.0;
+        if ((fl & FN_CH_ANGLE) && (st0 & 2)) {
+            if ((fl & FN_CH_AN_FL) && !(s_ok[tid - 1] && s_ok[tid])) {
+                st &= ~2u; /* kernel.cl:278-284 */
+            } else if (!FORCES_ONLY || (flags & FN_STEP_ANGLES)) {
+                const double* q = s_img + 3 * tid;
+                const double2 lp = s_len[tid - 1];
+                angle_arms(q[-3] - q[0], q[-2] - q[1], q[-1] - q[2], x, y, z, lp.x, lp.y, l, il, A.ch_an[i], pax, pay,
+                           paz, pcx, pcy, pcz);
+                cx = -pax - pcx;
+                cy = -pay - pcy;
+                cz = -paz - pcz;
+            }
         }
-        s_tan[u] = (unsigned char)alive;
-        if (alive && want_an) {
-            const int j = b0 - 1 + u;
-            const double* t1 = s_img + 3 * ((fl & FN_CH_AN_REV) ? u + 2 : u);
-            const double* t2 = s_img + 3 * (u + 1);
-            const double* t3 = s_img + 3 * ((fl & FN_CH_AN_REV) ? u : u + 2);
-            double* o = s_ang + 6 * u;
-            angle_pts(t1[0], t1[1], t1[2], t2[0], t2[1], t2[2], t3[0], t3[1], t3[2], A.ch_an[j],
-                      o[0], o[1], o[2], o[3], o[4], o[5]);
-        }
+        double* o = s_ang + 6 * tid;
+        o[0] = pax;
+        o[1] = pay;
+        o[2] = paz;
+        o[3] = pcx;
+        o[4] = pcy;
+        o[5] = pcz;
     }
     __syncthreads();
 
-    const bool active = tid < n;
-    const int i = b0 + tid;
-    const FnNet& N = A.nets[tile.net];
+    const bool active = tid >= 2 && tid < n + 2;
+    /* a block that stages this bead as halo may see the old status or the
+       new one: a bond that dies in this step acts in neither case */
+    if (!FORCES_ONLY && active && st != st0) A.ch_status[i] = (unsigned char)st;
+    const FnNet& N = UNIFORM ? A.net0 : A.nets[tile.net];
     double4 p = make_double4(0.0, 0.0, 0.0, 0.0);
     double Fx = 0.0, Fy = 0.0, Fz = 0.0;
     int nc = 0;
     if (active) {
         p = A.pos_in[i];
         if (!FORCES_ONLY) base_force<DAMP>(A, N, i, p, Fx, Fy, Fz);
-        if (want_sp) {
-            /* spring (i-1, i): bead i is p1 when the spring is reversed */
-            const unsigned fp = s_flag[tid + 1];
-            if ((fp & FN_CH_SPRING) && (s_tsp[tid + 1] & 1)) {
-                const double* f = s_spf + 3 * (tid + 1);
-                if (fp & FN_CH_SP_REV) {
-                    Fx += f[0];
-                    Fy += f[1];
-                    Fz += f[2];
-                } else {
-                    Fx += f[0] * -1.0;
-                    Fy += f[1] * -1.0;
-                    Fz += f[2] * -1.0;
-                }
-            }
-            /* spring (i, i+1): bead i is p1 unless reversed */
-            const unsigned fn = s_flag[tid + 2];
-            if ((fn & FN_CH_SPRING) && (s_tsp[tid + 2] & 1)) {
-                const double* f = s_spf + 3 * (tid + 2);
-                if (fn & FN_CH_SP_REV) {
-                    Fx += f[0] * -1.0;
-                    Fy += f[1] * -1.0;
-                    Fz += f[2] * -1.0;
-                } else {
-                    Fx += f[0];
-                    Fy += f[1];
-                    Fz += f[2];
-                }
-            }
-        }
-        if (want_an) {
-            /* centred on i-1: bead i is b3, or b1 when reversed */
-            if (s_tan[tid]) {
-                const double* o = s_ang + 6 * tid;
-                const int k = (s_flag[tid + 1] & FN_CH_AN_REV) ? 0 : 3;
-                Fx += o[k];
-                Fy += o[k + 1];
-                Fz += o[k + 2];
-            }
-            /* centred on i: bead i is b2 */
-            if (s_tan[tid + 1]) {
-                const double* o = s_ang + 6 * (tid + 1);
-                Fx += -o[0] - o[3];
-                Fy += -o[1] - o[4];
-                Fz += -o[2] - o[5];
-            }
-            /* centred on i+1: bead i is b1, or b3 when reversed */
-            if (s_tan[tid + 2]) {
-                const double* o = s_ang + 6 * (tid + 2);
-                const int k = (s_flag[tid + 3] & FN_CH_AN_REV) ? 3 : 0;
-                Fx += o[k];
-                Fy += o[k + 1];
-                Fz += o[k + 2];
-            }
-        }
-        if (!FORCES_ONLY || (terms & 4)) {
+        const double* f = s_spf + 3 * tid;
+        Fx -= f[-3];
+        Fy -= f[-2];
+        Fz -= f[-1];
+        Fx += f[0];
+        Fy += f[1];
+        Fz += f[2];
+        const double* o = s_ang + 6 * tid;
+        Fx += o[-3];
+        Fy += o[-2];
+        Fz += o[-1];
+        Fx += cx;
+        Fy += cy;
+        Fz += cz;
+        Fx += o[6];
+        Fy += o[7];
+        Fz += o[8];
+        if (!FORCES_ONLY || (flags & FN_STEP_CONTACTS)) {
             nc = A.list_count[i];
             if (nc > A.list_cap) nc = A.list_cap;
         }
@@ -720,12 +732,15 @@ __global__ void __launch_bounds__(kChainMaxBlock, 4) k_step_chain(const StepArgs
        involved. */
     {
         const int lane = tid & 31, wid = tid >> 5;
+        const int i0 = tile.begin - 2 + (tid & ~31); /* bead of the warp's lane 0 */
         unsigned char* s_map = smem_raw + L.wmap + 32 * (size_t)wid;
         double* s_R = reinterpret_cast<double*>(smem_raw + L.wres) + 3 * 32 * (size_t)wid;
         unsigned char* s_Rf = smem_raw + L.wresf + 32 * (size_t)wid;
-        const double4* s_pos = reinterpret_cast<const double4*>(smem_raw + L.pos);
-        double4* s_pos_w = reinterpret_cast<double4*>(smem_raw + L.pos);
-        if (active) s_pos_w[tid] = p;
+        double4* s_pos = reinterpret_cast<double4*>(smem_raw + L.pos) + (tid & ~31);
+        if (active) s_pos[lane] = p;
+        auto contact = [&](double4 a, double4 b, double& Rx, double& Ry, double& Rz) {
+            return UNIFORM ? contact_force(N, A.pair0, a, b, Rx, Ry, Rz) : contact_eval(N, A.pairs, a, b, Rx, Ry, Rz);
+        };
         /* direct phase: every lane first evaluates the leading KD items of its
            own list, one list row per iteration (coalesced loads, no window
            bookkeeping); the longer lists' tails then go through the windows.
@@ -765,16 +780,21 @@ __global__ void __launch_bounds__(kChainMaxBlock, 4) k_step_chain(const StepArgs
             __syncwarp();
             b_first = lane < lim ? s_map[lane] : 0;
             const int ob = __shfl_sync(0xffffffffu, off - nd, b_first);
-            if (lane < lim)
-                j_first = A.list[(size_t)(lane - ob) * A.list_stride + (b0 + (tid & ~31) + b_first)];
+            if (lane < lim) j_first = A.list[(size_t)(lane - ob) * A.list_stride + (i0 + b_first)];
         }
-        int jn = nd > 0 ? A.list[i] : 0; /* next list index, loaded one item ahead */
+        /* the next list index is loaded one item ahead, by every lane and
+           without a condition (a bead's own column, rows up to the list's
+           last): a conditional load is merged with the old value at once,
+           which waits for it */
+        const int* row = A.list + (active ? i : tile.begin);
+        int jn = *row;
         for (int k = 0; k < kd; ++k) {
+            const int j = jn;
+            if (k + 1 < A.list_cap) row += A.list_stride;
+            jn = *row;
             if (k < nd) {
-                const int j = jn;
-                if (k + 1 < nd) jn = A.list[(size_t)(k + 1) * A.list_stride + i];
                 double Rx = 0.0, Ry = 0.0, Rz = 0.0;
-                if (contact_eval(N, A.pairs, p, A.pos_in[j], Rx, Ry, Rz)) {
+                if (contact(p, A.pos_in[j], Rx, Ry, Rz)) {
                     Fx += Rx;
                     Fy += Ry;
                     Fz += Rz;
@@ -790,12 +810,11 @@ __global__ void __launch_bounds__(kChainMaxBlock, 4) k_step_chain(const StepArgs
                 __syncwarp();
                 b = w < lim ? s_map[lane] : 0;
                 const int ob = __shfl_sync(0xffffffffu, off - nd, b); /* list row = w - ob */
-                if (w < lim) j = A.list[(size_t)(w - ob) * A.list_stride + (b0 + (tid & ~31) + b)];
+                if (w < lim) j = A.list[(size_t)(w - ob) * A.list_stride + (i0 + b)];
             }
             if (w < lim) {
-                const int ib = (tid & ~31) + b; /* block-local bead of the item */
                 double Rx = 0.0, Ry = 0.0, Rz = 0.0;
-                const int acts = contact_eval(N, A.pairs, s_pos[ib], A.pos_in[j], Rx, Ry, Rz);
+                const int acts = contact(s_pos[b], A.pos_in[j], Rx, Ry, Rz);
                 s_R[3 * lane] = Rx;
                 s_R[3 * lane + 1] = Ry;
                 s_R[3 * lane + 2] = Rz;
@@ -817,13 +836,7 @@ __global__ void __launch_bounds__(kChainMaxBlock, 4) k_step_chain(const StepArgs
         A.force[i] = make_float4((float)Fx, (float)Fy, (float)Fz, 0.0f);
         return;
     }
-    /* statuses after this step (kernel.cl:396-397, 278-284) */
-    const unsigned st0 = s_stat[tid + 2];
-    unsigned st = st0;
-    if ((s_tsp[tid + 2] & 2)) st &= ~1u;
-    if ((st0 & 2) && (s_flag[tid + 2] & FN_CH_ANGLE) && !s_tan[tid + 1]) st &= ~2u;
-    if (st != st0) A.ch_status[i] = (unsigned char)st;
-    kick_drift_store<DAMP, DRIFT, STORE_V>(A, N, i, p, Fx, Fy, Fz);
+    kick_drift<DAMP>(A, N, i, p, Fx, Fy, Fz, (flags & FN_STEP_DRIFT) != 0, DAMP || (flags & FN_STEP_STORE_V));
 }
 
 /* ------------------------------------------------------------------------ */
@@ -2092,31 +2105,24 @@ __global__ void k_observe_final(const double* partial, int nblocks, double* out)
 /* ------------------------------------------------------------------------ */
 /* launch wrappers                                                           */
 
+static int step_flags(bool do_drift, bool store_v) {
+    return FN_STEP_SPRINGS | FN_STEP_ANGLES | FN_STEP_CONTACTS | (do_drift ? FN_STEP_DRIFT : 0) |
+           (store_v ? FN_STEP_STORE_V : 0);
+}
+
 cudaError_t launch_step(const StepArgs& A, int ntiles, int block, bool damp, bool do_drift,
                         bool store_v, cudaStream_t s) {
     if (ntiles <= 0) return cudaSuccess;
-    if (damp) {
-        if (do_drift)
-            k_step<true, true, true><<<ntiles, block, 0, s>>>(A);
-        else
-            k_step<true, false, false><<<ntiles, block, 0, s>>>(A);
-    } else {
-        if (do_drift) {
-            if (store_v)
-                k_step<false, true, true><<<ntiles, block, 0, s>>>(A);
-            else
-                k_step<false, true, false><<<ntiles, block, 0, s>>>(A);
-        } else {
-            k_step<false, false, false><<<ntiles, block, 0, s>>>(A);
-        }
-    }
+    if (damp)
+        k_step<true><<<ntiles, block, 0, s>>>(A, step_flags(do_drift, store_v));
+    else
+        k_step<false><<<ntiles, block, 0, s>>>(A, step_flags(do_drift, store_v));
     return cudaGetLastError();
 }
 
-template <bool DAMP, bool DRIFT, bool STORE_V>
+template <bool DAMP, bool UNI>
 static cudaError_t set_tiled_smem(size_t bytes) {
-    return cudaFuncSetAttribute(k_step_tiled<DAMP, DRIFT, STORE_V>,
-                                cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    return cudaFuncSetAttribute(k_step_tiled<DAMP, UNI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
 }
 
 /* The dynamic shared-memory limit is an attribute of the kernel on a
@@ -2134,72 +2140,57 @@ cudaError_t prepare_step_tiled(size_t bytes) {
     static size_t done[64] = {};
     if (!raise_limit(done, bytes)) return cudaSuccess;
     cudaError_t e;
-    if ((e = set_tiled_smem<true, true, true>(bytes))) return e;
-    if ((e = set_tiled_smem<true, false, false>(bytes))) return e;
-    if ((e = set_tiled_smem<false, true, true>(bytes))) return e;
-    if ((e = set_tiled_smem<false, true, false>(bytes))) return e;
-    return set_tiled_smem<false, false, false>(bytes);
+    if ((e = set_tiled_smem<true, true>(bytes))) return e;
+    if ((e = set_tiled_smem<true, false>(bytes))) return e;
+    if ((e = set_tiled_smem<false, true>(bytes))) return e;
+    return set_tiled_smem<false, false>(bytes);
 }
 
 cudaError_t launch_step_tiled(const StepArgs& A, int ntiles, int block, bool damp, bool do_drift,
                               bool store_v, cudaStream_t s) {
     if (ntiles <= 0) return cudaSuccess;
     const size_t sm = step_tiled_smem(A.max_tile_sp, A.max_tile_an);
-    if (damp) {
-        if (do_drift)
-            k_step_tiled<true, true, true><<<ntiles, block, sm, s>>>(A);
-        else
-            k_step_tiled<true, false, false><<<ntiles, block, sm, s>>>(A);
-    } else {
-        if (do_drift) {
-            if (store_v)
-                k_step_tiled<false, true, true><<<ntiles, block, sm, s>>>(A);
-            else
-                k_step_tiled<false, true, false><<<ntiles, block, sm, s>>>(A);
-        } else {
-            k_step_tiled<false, false, false><<<ntiles, block, sm, s>>>(A);
-        }
-    }
+    const int flags = step_flags(do_drift, store_v);
+    if (damp && A.uniform)
+        k_step_tiled<true, true><<<ntiles, block, sm, s>>>(A, flags);
+    else if (damp)
+        k_step_tiled<true, false><<<ntiles, block, sm, s>>>(A, flags);
+    else if (A.uniform)
+        k_step_tiled<false, true><<<ntiles, block, sm, s>>>(A, flags);
+    else
+        k_step_tiled<false, false><<<ntiles, block, sm, s>>>(A, flags);
     return cudaGetLastError();
 }
 
-template <bool DAMP, bool DRIFT, bool STORE_V, bool FO>
+template <bool DAMP, bool FO, bool UNI>
 static cudaError_t set_chain_smem(size_t bytes) {
-    return cudaFuncSetAttribute(k_step_chain<DAMP, DRIFT, STORE_V, FO>,
-                                cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    return cudaFuncSetAttribute(k_step_chain<DAMP, FO, UNI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
 }
 
 cudaError_t prepare_step_chain(size_t bytes) {
     static size_t done[64] = {};
     if (!raise_limit(done, bytes)) return cudaSuccess;
     cudaError_t e;
-    if ((e = set_chain_smem<true, true, true, false>(bytes))) return e;
-    if ((e = set_chain_smem<true, false, false, false>(bytes))) return e;
-    if ((e = set_chain_smem<false, true, true, false>(bytes))) return e;
-    if ((e = set_chain_smem<false, true, false, false>(bytes))) return e;
-    if ((e = set_chain_smem<false, false, false, false>(bytes))) return e;
-    return set_chain_smem<false, false, false, true>(bytes);
+    if ((e = set_chain_smem<true, false, false>(bytes))) return e;
+    if ((e = set_chain_smem<true, false, true>(bytes))) return e;
+    if ((e = set_chain_smem<false, false, false>(bytes))) return e;
+    if ((e = set_chain_smem<false, false, true>(bytes))) return e;
+    return set_chain_smem<false, true, false>(bytes);
 }
 
 cudaError_t launch_step_chain(const StepArgs& A, int ntiles, int block, bool damp, bool do_drift,
                               bool store_v, cudaStream_t s) {
     if (ntiles <= 0) return cudaSuccess;
     const size_t sm = step_chain_smem(block);
-    if (damp) {
-        if (do_drift)
-            k_step_chain<true, true, true, false><<<ntiles, block, sm, s>>>(A, 0);
-        else
-            k_step_chain<true, false, false, false><<<ntiles, block, sm, s>>>(A, 0);
-    } else {
-        if (do_drift) {
-            if (store_v)
-                k_step_chain<false, true, true, false><<<ntiles, block, sm, s>>>(A, 0);
-            else
-                k_step_chain<false, true, false, false><<<ntiles, block, sm, s>>>(A, 0);
-        } else {
-            k_step_chain<false, false, false, false><<<ntiles, block, sm, s>>>(A, 0);
-        }
-    }
+    const int flags = step_flags(do_drift, store_v);
+    if (damp && A.uniform)
+        k_step_chain<true, false, true><<<ntiles, block, sm, s>>>(A, flags);
+    else if (damp)
+        k_step_chain<true, false, false><<<ntiles, block, sm, s>>>(A, flags);
+    else if (A.uniform)
+        k_step_chain<false, false, true><<<ntiles, block, sm, s>>>(A, flags);
+    else
+        k_step_chain<false, false, false><<<ntiles, block, sm, s>>>(A, flags);
     return cudaGetLastError();
 }
 
@@ -2245,7 +2236,7 @@ cudaError_t launch_step_staged(const StepArgs& A, int ntiles, int block, bool da
 
 cudaError_t launch_forces_chain(const StepArgs& A, int ntiles, int block, int terms, cudaStream_t s) {
     if (ntiles <= 0) return cudaSuccess;
-    k_step_chain<false, false, false, true><<<ntiles, block, step_chain_smem(block), s>>>(A, terms);
+    k_step_chain<false, true, false><<<ntiles, block, step_chain_smem(block), s>>>(A, terms);
     return cudaGetLastError();
 }
 

@@ -68,6 +68,11 @@ struct StepArgs {
     long long csr_region;
     const int* tile_items;
     int chunk; /* contact items staged per round (a multiple of the block size) */
+    /* one network with one pair law for all bead types: both by value, so
+       that the chain kernel reads them as constants */
+    int uniform;
+    FnNet net0;
+    FnPair pair0;
 };
 
 /* dynamic shared memory of the tiled step kernel */
@@ -91,40 +96,35 @@ enum {
 };
 
 /* Byte offsets of the chain step kernel's dynamic shared memory for blocks
-   of `block` threads (one layout for host sizing and device carving). */
+   of `block` threads (one layout for host sizing and device carving).  Slot u
+   belongs to bead tile begin - 2 + u. */
 struct ChainSmem {
-    size_t img, spf, ang, flag, stat, tsp, tan, pos, wres, wmap, wresf, total;
+    size_t img, len, spf, ang, ok, pos, wres, wmap, wresf, total;
 };
 
 __host__ __device__ inline size_t smem_align(size_t o, size_t a) { return (o + a - 1) / a * a; }
 
 __host__ __device__ inline ChainSmem chain_smem_layout(int block) {
     ChainSmem L;
-    const size_t h = (size_t)block + 4;
+    const size_t h = (size_t)block;
     size_t o = 0;
-    L.img = o;  /* image positions of beads b0-2 .. b0+n+1, 3 doubles each */
+    L.img = o; /* image positions, 3 doubles each */
     o += 24 * h;
-    L.spf = o;  /* spring forces, lower bead b0-2 .. b0+n */
+    L.len = o; /* distance to the next bead and its inverse */
+    o += 16 * h;
+    L.pos = L.img; /* wrapped positions (double4), once the bonds are done */
+    L.spf = o;     /* force on the lower bead of spring (u, u + 1) */
     o += 24 * h;
-    L.ang = o;  /* angle pa, pc, centre b0-1 .. b0+n */
+    L.ang = o; /* angle centred on u: force on u - 1, on u + 1 */
     o += 48 * h;
-    L.flag = o; /* bead flags */
-    o += h;
-    L.stat = o; /* bead statuses */
-    o += h;
-    L.tsp = o;  /* spring term flags */
-    o += h;
-    L.tan = o;  /* angle term flags */
-    o += h;
-    o = smem_align(o, 32);
-    L.pos = o;  /* own wrapped positions, double4 */
-    o += 32 * (size_t)block;
     L.wres = o; /* per warp: contact results of one window of 32 items */
-    o += 24 * (size_t)block;
+    o += 24 * h;
     L.wmap = o; /* per warp: item -> lane map of the window */
-    o += (size_t)block;
+    o += h;
     L.wresf = o; /* per warp: result flags */
-    o += (size_t)block;
+    o += h;
+    L.ok = o; /* spring (u, u + 1) alive after this step */
+    o += h;
     L.total = smem_align(o, 16);
     return L;
 }

@@ -39,9 +39,13 @@ struct FnNet {
                            cut-off, plus the Verlet skin in displacement mode */
 };
 
-/* Pair coefficients c1..c6 (SimulationManager.cpp:891-932) and kind. */
+/* Pair coefficients c1..c6 (SimulationManager.cpp:891-932) and kind; for lj
+   also sigma^2 and 48 epsilon, and the smallest squared distance the shared-
+   seed arithmetic of the step kernels takes (infinity when the coefficients
+   are so large or small that an intermediate could leave the normal range). */
 struct FnPair {
     double c[6];
+    double lj_s2, lj_e48, lj_r2_min;
     int kind;
     int pad_;
 };

@@ -168,11 +168,15 @@ __device__ __forceinline__ void angle_eval(const StepArgs& A, int4 b, float2 par
 
 /* One contact-list entry (kernel.cl:835-999) under the pair law P: force on
    bead i.  Roots, reciprocals and quotients of the distance share one seed
-   (fn_rounded.cuh); distances outside its range take the operators. */
-__device__ __forceinline__ int contact_force(const FnNet& N, const FnPair& law, double4 pi, double4 pj, double& Rx,
-                                             double& Ry, double& Rz) {
+   (fn_rounded.cuh); distances outside its range take the operators.  Also the
+   separation (rx, ry, rz), the distance r and its inverse of an acting pair. */
+__device__ __forceinline__ int contact_law(const FnNet& N, const FnPair& law, double4 pi, double4 pj, double& Rx,
+                                           double& Ry, double& Rz, double& rx, double& ry, double& rz, double& r,
+                                           double& ir) {
     const FnPair* P = &law;
-    double rx = pi.x - pj.x, ry = pi.y - pj.y, rz = pi.z - pj.z;
+    rx = pi.x - pj.x;
+    ry = pi.y - pj.y;
+    rz = pi.z - pj.z;
     double length = rx * rx + ry * ry + rz * rz;
     length = min_image(N, rx, ry, rz, length, N.force_mi);
     const int kind = P->kind;
@@ -195,49 +199,55 @@ __device__ __forceinline__ int contact_force(const FnNet& N, const FnPair& law, 
             const double fr2 = P->lj_s2 / r2;
             const double fr6 = fr2 * fr2 * fr2;
             fpr = P->lj_e48 * fr6 * (fr6 - 0.5) / r2;
-            length = (length != 0.0) ? 1.0 / length : 0.0;
+            ir = (r != 0.0) ? 1.0 / r : 0.0;
         }
         fpr -= P->c[3];
-        Rx = fpr * (rx * length);
-        Ry = fpr * (ry * length);
-        Rz = fpr * (rz * length);
+        Rx = fpr * (rx * ir);
+        Ry = fpr * (ry * ir);
+        Rz = fpr * (rz * ir);
         return 1;
     }
-    double mag, inv;
+    double mag;
     if (kind == 2) {
-        root_and_inverse(length, length, inv);
-        mag = ((double)w_radius(pi.w) + (double)w_radius(pj.w)) - length;
+        root_and_inverse(length, r, ir);
+        mag = ((double)w_radius(pi.w) + (double)w_radius(pj.w)) - r;
         if (!(mag > 0.0)) return 0;
         mag *= P->c[0];
     } else if (kind == 4) {
         /* extension, no counterpart in the reference: penalty spring K (c1)
            on the overlap plus a soft harmonic repulsion k (c2) below rc (c3) */
-        root_and_inverse(length, length, inv);
-        const double penetration = ((double)w_radius(pi.w) + (double)w_radius(pj.w)) - length;
+        root_and_inverse(length, r, ir);
+        const double penetration = ((double)w_radius(pi.w) + (double)w_radius(pj.w)) - r;
         mag = 0.0;
         int acts = 0;
         if (penetration > 0.0) {
             mag += penetration * P->c[0];
             acts = 1;
         }
-        if (length < P->c[2]) {
-            mag += (P->c[2] - length) * P->c[1];
+        if (r < P->c[2]) {
+            mag += (P->c[2] - r) * P->c[1];
             acts = 1;
         }
         if (!acts) return 0;
     } else if (kind == 3) {
         if (!(length < P->c[3])) return 0;
-        root_and_inverse(length, length, inv);
-        mag = (P->c[1] - length);
+        root_and_inverse(length, r, ir);
+        mag = (P->c[1] - r);
         mag *= P->c[0]; /* both arms of kernel.cl:970-973 multiply by K */
-        mag += (P->c[5] - length) * P->c[4];
+        mag += (P->c[5] - r) * P->c[4];
     } else {
         return 0;
     }
-    Rx = mag * (rx * inv);
-    Ry = mag * (ry * inv);
-    Rz = mag * (rz * inv);
+    Rx = mag * (rx * ir);
+    Ry = mag * (ry * ir);
+    Rz = mag * (rz * ir);
     return 1;
+}
+
+__device__ __forceinline__ int contact_force(const FnNet& N, const FnPair& law, double4 pi, double4 pj, double& Rx,
+                                             double& Ry, double& Rz) {
+    double rx, ry, rz, r, ir;
+    return contact_law(N, law, pi, pj, Rx, Ry, Rz, rx, ry, rz, r, ir);
 }
 
 /* The same with the law looked up by the beads' types. */
@@ -2094,12 +2104,24 @@ __global__ void k_observe_partial(const ObserveArgs O) {
     }
 }
 
+/* The sum over the blocks' partial sums of quantity `warp` of NQ, one warp per
+   quantity: lane l adds blocks l, l + 32, ... and the lanes are added by
+   halves, a fixed order.  (One thread adding up to 1,024 x 5 doubles one
+   after the other took 197 us, 13x the partial sums themselves.) */
+template <int NQ>
+__device__ __forceinline__ void add_partials(const double* partial, int nblocks, double* out) {
+    const int lane = threadIdx.x & 31, k = threadIdx.x >> 5;
+    if (k >= NQ) return;
+    double a = 0.0;
+#pragma unroll 8
+    for (int b = lane; b < nblocks; b += 32) a += partial[NQ * (size_t)b + k];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) a += __shfl_down_sync(0xffffffffu, a, o);
+    if (lane == 0) out[k] = a;
+}
+
 __global__ void k_observe_final(const double* partial, int nblocks, double* out) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    double a[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
-    for (int b = 0; b < nblocks; ++b)
-        for (int k = 0; k < 5; ++k) a[k] += partial[5 * (size_t)b + k];
-    for (int k = 0; k < 5; ++k) out[k] = a[k];
+    add_partials<5>(partial, nblocks, out);
 }
 
 /* ------------------------------------------------------------------------ */
@@ -2386,21 +2408,16 @@ __device__ __forceinline__ double contact_energy(const FnNet& N, const FnPair* _
                                                  double4 pi, double4 pj, double& Rx, double& Ry,
                                                  double& Rz, double& rx, double& ry, double& rz,
                                                  int& acts) {
-    rx = pi.x - pj.x;
-    ry = pi.y - pj.y;
-    rz = pi.z - pj.z;
-    double r2 = rx * rx + ry * ry + rz * rz;
-    r2 = min_image(N, rx, ry, rz, r2, N.force_mi);
-    acts = contact_eval(N, pairs, pi, pj, Rx, Ry, Rz);
-    if (!acts) return 0.0;
     const FnPair* P = pairs + N.pair_base + getadress(w_type(pi.w), w_type(pj.w), N.types_num);
-    const double r = sqrt(r2);
+    double r, ir;
+    acts = contact_law(N, *P, pi, pj, Rx, Ry, Rz, rx, ry, rz, r, ir);
+    if (!acts) return 0.0;
     const double rsum = (double)w_radius(pi.w) + (double)w_radius(pj.w);
     switch (P->kind) {
     case 1: {
         const double rc = P->c[2], s2 = P->c[0] * P->c[0], eps = P->c[1];
         const double s6 = s2 * s2 * s2, s12 = s6 * s6;
-        const double ir = 1.0 / r, irc = 1.0 / rc;
+        const double irc = 1.0 / rc;
         /* r^-7 and r^-13 by products (within a few ulp of pow, far cheaper) */
         const double ir2 = ir * ir, ir6 = ir2 * ir2 * ir2, ir7 = ir6 * ir, ir13 = ir6 * ir7;
         const double irc2 = irc * irc, irc6 = irc2 * irc2 * irc2, irc7 = irc6 * irc, irc13 = irc6 * irc7;
@@ -2444,7 +2461,7 @@ __device__ __forceinline__ void add_outer(double* w, double ax, double ay, doubl
    hide (measured on the 1M-bead tensile network: 0.37 ms per evaluation
    against 0.45 ms at the 102 registers the compiler picks unbounded). */
 __global__ void __launch_bounds__(256, 3) k_energy_partial(const EnergyArgs E) {
-    __shared__ double red[256];
+    __shared__ double red[8][FN_EN_N];
     const FnNet& N = E.nets[E.net];
     double acc[FN_EN_N];
 #pragma unroll
@@ -2523,36 +2540,38 @@ __global__ void __launch_bounds__(256, 3) k_energy_partial(const EnergyArgs E) {
         add_outer(W, bax, bay, baz, pax, pay, paz);
         add_outer(W, bcx, bcy, bcz, pcx, pcy, pcz);
     }
-    /* fixed-order block reduction, one quantity at a time */
+    /* fixed-order block reduction: each warp by halves, then the warps in
+       order (the block-wide tree, a barrier per halving and quantity, was a
+       third of the kernel on a 100k-bead network) */
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
     for (int k = 0; k < FN_EN_N; ++k) {
-        red[threadIdx.x] = acc[k];
-        __syncthreads();
-        for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-            if (threadIdx.x < o) red[threadIdx.x] += red[threadIdx.x + o];
-            __syncthreads();
-        }
-        if (threadIdx.x == 0) E.partial[(size_t)FN_EN_N * blockIdx.x + k] = red[0];
-        __syncthreads();
+        double a = acc[k];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) a += __shfl_down_sync(0xffffffffu, a, o);
+        if (lane == 0) red[warp][k] = a;
+    }
+    __syncthreads();
+    if (threadIdx.x < FN_EN_N) {
+        double a = 0.0;
+        for (int w = 0; w < 8; ++w) a += red[w][threadIdx.x];
+        E.partial[(size_t)FN_EN_N * blockIdx.x + threadIdx.x] = a;
     }
 }
 
 __global__ void k_energy_final(const double* partial, int nblocks, double* out) {
-    const int k = threadIdx.x;
-    if (blockIdx.x != 0 || k >= FN_EN_N) return;
-    double a = 0.0;
-    for (int b = 0; b < nblocks; ++b) a += partial[(size_t)FN_EN_N * b + k];
-    out[k] = a;
+    add_partials<FN_EN_N>(partial, nblocks, out);
 }
 
 cudaError_t launch_energy(const EnergyArgs& E, int nblocks, double* out, cudaStream_t s) {
     k_energy_partial<<<nblocks, 256, 0, s>>>(E);
-    k_energy_final<<<1, 32, 0, s>>>(E.partial, nblocks, out);
+    k_energy_final<<<1, 32 * FN_EN_N, 0, s>>>(E.partial, nblocks, out);
     return cudaGetLastError();
 }
 
 cudaError_t launch_observe(const ObserveArgs& O, int nblocks, double* out, cudaStream_t s) {
     k_observe_partial<<<nblocks, 256, 0, s>>>(O);
-    k_observe_final<<<1, 32, 0, s>>>(O.partial, nblocks, out);
+    k_observe_final<<<1, 32 * 5, 0, s>>>(O.partial, nblocks, out);
     return cudaGetLastError();
 }
 

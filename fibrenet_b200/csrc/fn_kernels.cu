@@ -186,16 +186,16 @@ __device__ __forceinline__ int contact_law(const FnNet& N, const FnPair& law, do
         double fpr;
         if (r2 >= P->lj_r2_min) {
             const double y = rsqrt_seeded(r2);
-            const double r = root_from(r2, y);
+            r = root_from(r2, y);
             if (!(r < P->c[2])) return 0;
-            length = recip_from(r, y);
+            ir = recip_from(r, y);
             const double ir2 = recip_from(r2, y * y);
             const double fr2 = quotient(P->lj_s2, r2, ir2);
             const double fr6 = fr2 * fr2 * fr2;
             fpr = quotient(P->lj_e48 * fr6 * (fr6 - 0.5), r2, ir2);
         } else {
-            length = sqrt(length);
-            if (!(length < P->c[2])) return 0;
+            r = sqrt(r2);
+            if (!(r < P->c[2])) return 0;
             const double fr2 = P->lj_s2 / r2;
             const double fr6 = fr2 * fr2 * fr2;
             fpr = P->lj_e48 * fr6 * (fr6 - 0.5) / r2;

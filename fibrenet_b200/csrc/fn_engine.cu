@@ -51,6 +51,52 @@ double list_r2(const NetHost& h, double cutoff_sq, double smax) {
     return r2;
 }
 
+/* The listing radii of network N, for the list build: list_r2_max, beyond
+   which no pair is listed, and the same from positions rounded to FP32 (smax:
+   largest skin radius, rmin and smin: smallest radius and skin radius).  An
+   axis of a separation is then off by less than 4 B 2^-24 (B the longest box
+   side: two positions, their difference, the box side of a wrapped neighbour),
+   the distance by less than 8 B 2^-24, and its square by 2^-21 of itself.
+   The FP32 test moves the bead by the box for cells beyond a periodic side
+   and leaves the others where they are.  That is what the minimum image does
+   to every pair within the radius when the box is longer than the radius and
+   two cells (a pair in neighbouring cells is at most two cells apart), and to
+   every pair when moreover two cells are less than half of the shortest side
+   and the box longer than four cells. */
+void set_list_radii(FnNet& N, const NetHost& h, double smax, double rmin, double smin) {
+    N.list_r2_max = list_r2(h, N.list_cut_sq, smax);
+    const double err = std::max({N.box[0], N.box[1], N.box[2]}) * std::ldexp(1.0, -21);
+    const double shortest = std::min({N.box[0], N.box[1], N.box[2]});
+    const double out = std::sqrt(N.list_r2_max) + err;
+    const double cut = std::sqrt(N.list_cut_sq), hs = rmin + smin;
+    double in = 1e300;
+    if (h.kinds & (1u << FN_PAIR_LJ | 1u << FN_PAIR_ST)) in = cut;
+    if (h.kinds & 1u << FN_PAIR_HS) in = std::min(in, hs);
+    if (h.kinds & 1u << FN_PAIR_HSR) in = std::min(in, std::max(cut, hs));
+    in -= err;
+    bool out_ok = out < 1e15, in_ok = in > 0.0 && in < 1e15 && !(h.kinds & 1u);
+    for (int a = 0; a < 3; ++a) {
+        if (!(N.list_mi >> a & 1)) continue;
+        out_ok = out_ok && N.box[a] - 2.0 * N.step[a] > 1.001 * out;
+        in_ok = in_ok && 2.001 * N.step[a] < 0.5 * shortest && N.box[a] > 4.001 * N.step[a];
+    }
+    N.list_out_r2 = out_ok ? std::nextafter((float)(out * out * (1.0 + 1e-6)), std::numeric_limits<float>::infinity()) : -1.0f;
+    N.list_in_r2 = out_ok && in_ok ? std::nextafter((float)(in * in * (1.0 - 1e-6)), 0.0f) : -1.0f;
+}
+
+/* the skin radius the upload gives a bead */
+double skin_of(double radius, double skin_ratio) { return (double)(float)(radius + skin_ratio); }
+
+/* c / d = umulhi(c, mul) >> shift for every c < 2^31 (d >= 2): with
+   2^l >= d > 2^(l-1), mul = ceil(2^(31+l) / d) is off by less than one in d,
+   which c 2^-(31+l) keeps below 1/d. */
+void division(int d, unsigned& mul, int& shift) {
+    int l = 1;
+    while ((1ll << l) < d) ++l;
+    mul = (unsigned)(((1ull << (31 + l)) + (unsigned long long)d - 1) / (unsigned long long)d);
+    shift = l - 1;
+}
+
 uint32_t spread10(uint32_t v) {
     v &= 0x3ff;
     v = (v | (v << 16)) & 0x030000FF;
@@ -227,6 +273,8 @@ void free_all(fn_ctx* c) {
     dfree(c, c->cell_fill);
     dfree(c, c->cell_start);
     dfree(c, c->cell_beads);
+    dfree(c, c->cell_raw);
+    dfree(c, c->cell_pos);
     dfree(c, c->ref_img);
     dfree(c, c->inv_d);
     dfree(c, c->perm_d);
@@ -307,6 +355,8 @@ int derive_net(fn_ctx* c, const fn_settings& s, FnNet& N, int net_index) {
         N.force_mi = N.periodic;
         N.walls = (~N.periodic) & 7;
     }
+    division(N.nx, N.div_nx, N.shift_nx);
+    division(N.nxy, N.div_nxy, N.shift_nxy);
     N.types_num = s.n_types;
     return FN_OK;
 }
@@ -876,6 +926,13 @@ fn::RebuildArgs rebuild_args(fn_ctx* c) {
     R.cell_fill = c->cell_fill.p;
     R.cell_start = c->cell_start.p;
     R.cell_beads = c->cell_beads.p;
+    R.cell_raw = c->cell_raw.p;
+    R.cell_pos = c->cell_pos.p;
+    R.uniform = c->uniform ? 1 : 0;
+    if (c->uniform) {
+        R.net0 = c->nets_h[0];
+        R.pair0 = c->pairs_h[0];
+    }
     R.gate = c->verlet ? c->gate.p : nullptr;
     R.list_count = c->list_count.p;
     R.list = c->list.p;
@@ -1180,6 +1237,7 @@ static int net_preamble(fn_ctx* c, int k, const fn_network_desc& d, long long& n
     const int npairs = nt * (nt + 1) / 2;
     N.pair_base = (int)c->pairs_h.size();
     bool any_cut = false, any_hs = false;
+    unsigned kinds = 0;
     for (int p = 0; p < npairs; ++p) {
         FnPair P;
         pair_coeffs(d.pair_kind[p], d.pair_raw + 4 * p, P);
@@ -1189,23 +1247,26 @@ static int net_preamble(fn_ctx* c, int k, const fn_network_desc& d, long long& n
         c->pairs_h.push_back(P);
         any_cut |= P.kind == FN_PAIR_LJ || P.kind == FN_PAIR_ST || P.kind == FN_PAIR_HSR;
         any_hs |= P.kind == FN_PAIR_HS || P.kind == FN_PAIR_HSR;
+        kinds |= 1u << (P.kind >= FN_PAIR_LJ && P.kind <= FN_PAIR_HSR ? P.kind : 0);
     }
     /* largest listing radius (squared): cutoff for lj/st, the largest
        radius + the largest skin for hs (kernel.cl:632-650) */
-    double rmax = 0.0, smax = 0.0, gap = 1e300;
+    double rmax = 0.0, smax = 0.0, gap = 1e300, rmin = 1e300;
     std::mutex red;
     if (element_checks)
         parallel_for(d.n_beads, [&](long long i0, long long i1) {
-        double r = 0.0, sm = 0.0, g = 1e300;
+        double r = 0.0, sm = 0.0, g = 1e300, lo = 1e300;
         for (long long i = i0; i < i1; ++i) {
             const float rad = (float)d.radius[i];
             const float skin = (float)((double)rad + d.settings.skin_ratio);
             r = std::max(r, (double)rad);
+            lo = std::min(lo, (double)rad);
             sm = std::max(sm, (double)skin);
             g = std::min(g, (double)skin - (double)rad);
         }
         std::lock_guard<std::mutex> lk(red);
         rmax = std::max(rmax, r);
+        rmin = std::min(rmin, lo);
         smax = std::max(smax, sm);
         gap = std::min(gap, g);
     });
@@ -1213,7 +1274,8 @@ static int net_preamble(fn_ctx* c, int k, const fn_network_desc& d, long long& n
     c->info[k].any_cut = any_cut;
     c->info[k].any_hs = any_hs;
     c->info[k].rmax = rmax;
-    N.list_r2_max = list_r2(c->info[k], N.list_cut_sq, smax);
+    c->info[k].kinds = kinds;
+    set_list_radii(N, c->info[k], smax, rmin, skin_of(rmin, d.settings.skin_ratio));
     NetHost& h = c->info[k];
     h.bead_begin = (int)nb;
     h.bead_end = (int)(nb + d.n_beads);
@@ -1243,10 +1305,11 @@ static int net_preamble(fn_ctx* c, int k, const fn_network_desc& d, long long& n
 
 /* largest radius, largest skin radius and smallest skin - radius of network
    k: the listing radius of its hs pairs and the displacement threshold */
-static void set_radius_extremes(fn_ctx* c, int k, double rmax, double smax, double gap) {
+static void set_radius_extremes(fn_ctx* c, int k, double rmax, double smax, double gap, double rmin,
+                                double skin_ratio) {
     c->info[k].skin_gap = gap;
     c->info[k].rmax = rmax;
-    c->nets_h[k].list_r2_max = list_r2(c->info[k], c->nets_h[k].list_cut_sq, smax);
+    set_list_radii(c->nets_h[k], c->info[k], smax, rmin, skin_of(rmin, skin_ratio));
 }
 
 /* The context's device buffers for a model of these sizes, whichever path
@@ -1283,6 +1346,8 @@ static cudaError_t alloc_model(fn_ctx* c, long long nb, long long ns, long long 
     AL(dalloc(c, c->cell_fill, ncells));
     AL(dalloc(c, c->cell_start, ncells + 1));
     AL(dalloc(c, c->cell_beads, nb));
+    AL(dalloc(c, c->cell_raw, nb));
+    AL(dalloc(c, c->cell_pos, nb));
     AL(dalloc(c, c->list_count, nb));
     AL(dalloc(c, c->list, list_n));
     AL(dalloc(c, c->scan_sums, (size_t)std::max(fn::scan_block_count(ncells), fn::scan_block_count(nb)) + 1));
@@ -1584,7 +1649,7 @@ static int upload_device(fn_ctx* c, int n_networks, const fn_network_desc* nets)
         chk[k].bad_bead = chk[k].bad_spring = chk[k].bad_angle = 0x7fffffff;
         chk[k].not_runs = 0;
         chk[k].rmax = chk[k].smax = 0ull;
-        chk[k].gmin = ~0ull;
+        chk[k].gmin = chk[k].rmin = ~0ull;
     }
     /* the caller's arrays, network by network */
     for (int k = 0; k < n_networks; ++k) {
@@ -1699,7 +1764,8 @@ static int upload_device(fn_ctx* c, int n_networks, const fn_network_desc* nets)
         const fn::UpCheck& q = chk[k];
         if (q.bad_bead != 0x7fffffff || q.bad_spring != 0x7fffffff || q.bad_angle != 0x7fffffff || q.not_runs)
             return kUploadFallback;
-        set_radius_extremes(c, k, undkey(q.rmax), undkey(q.smax), undkey(q.gmin));
+        set_radius_extremes(c, k, undkey(q.rmax), undkey(q.smax), undkey(q.gmin), undkey(q.rmin),
+                            nets[k].settings.skin_ratio);
     }
 
     /* bead order: the runs (fibres) of each network sorted by key, as the
@@ -2023,15 +2089,18 @@ FN_API int fn_set_skin(fn_ctx* c, const double* skin) {
     }
     for (int k = 0; k < c->n_nets; ++k) {
         double smax = 0.0;
-        double gap = 1e300;
+        double gap = 1e300, rmin = 1e300, smin = 1e300;
         for (int i = c->info[k].bead_begin; i < c->info[k].bead_end; ++i) {
             smax = std::max(smax, (double)(float)skin[i]);
             gap = std::min(gap, (double)(float)skin[i] - (double)radius[i]);
+            rmin = std::min(rmin, (double)radius[i]);
+            smin = std::min(smin, (double)(float)skin[i]);
         }
         c->info[k].skin_gap = gap;
-        c->nets_h[k].list_r2_max = list_r2(c->info[k], c->nets_h[k].list_cut_sq, smax);
+        set_list_radii(c->nets_h[k], c->info[k], smax, rmin, smin);
     }
     CK(cudaMemcpy(c->nets.p, c->nets_h.data(), sizeof(FnNet) * c->n_nets, cudaMemcpyHostToDevice));
+    drop_graphs(c); /* captured rebuilds carry the listing radius */
     r = verlet_setup(c);
     if (r) return r;
     return FN_OK;

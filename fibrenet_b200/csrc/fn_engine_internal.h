@@ -39,6 +39,7 @@ struct NetHost {
     int grid_update_freq;
     double damping;
     bool any_cut, any_hs; /* pair kinds present (listing radius) */
+    unsigned kinds;       /* bit k: some type pair is of kind k (bit 0: of a kind that lists nothing) */
     double rmax;          /* largest radius, as stored */
     double skin_gap;      /* smallest skin radius - radius over the beads */
 };
@@ -105,8 +106,9 @@ struct fn_ctx {
     long long csr_region = 0;
     DevBuf<int> csr, tile_items;
     DevBuf<int> cell_of, cell_count, cell_fill, cell_start, cell_beads, list_count, list;
+    DevBuf<float4> cell_raw, cell_pos;
     DevBuf<int> scan_sums;
-    /* the list build: 0 one thread per bead (the default), 1 by bricks of
+    /* the list build: 0 bead by bead (the default), 1 by bricks of
        cells (network, first cell x, y, z of each) staged in shared memory,
        2 by groups of 8 lanes per bead */
     DevBuf<int4> bricks;

@@ -1308,58 +1308,87 @@ __global__ void k_cells(const RebuildArgs R) {
     R.list_count[i] = 0; /* k_lists counts only the beads it lists */
 }
 
-__global__ void k_scatter(const RebuildArgs R, int nb) {
+/* FillGrid's slot of each bead in its cell: the bead as the list build's first
+   test reads it, 16 bytes with its position rounded to FP32 and its index. */
+__global__ void k_scatter(const __grid_constant__ RebuildArgs R, int nb) {
     FN_GATED(R.gate);
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= nb) return;
     const int c = R.cell_of[i];
     if (c < 0) return;
+    const double4 p = R.pos[i];
     const int slot = atomicAdd(R.cell_fill + c, 1);
-    R.cell_beads[R.cell_start[c] + slot] = i;
+    R.cell_raw[R.cell_start[c] + slot] = make_float4((float)p.x, (float)p.y, (float)p.z, __int_as_float(i));
+}
+
+/* The first n <= W beads of a cell by index: Batcher's network for W = 4 or 8
+   on (index, slot) keys in registers, absent slots last. */
+template <int W>
+__device__ __forceinline__ void cell_sort_small(const float4* raw, int n, int* b, float4* e) {
+    constexpr int N4 = 5, N8 = 19;
+    constexpr int net[N8][2] = {{0, 1}, {2, 3}, {0, 2}, {1, 3}, {1, 2}, {4, 5}, {6, 7}, {4, 6}, {5, 7}, {5, 6},
+                                {0, 4}, {1, 5}, {2, 6}, {3, 7}, {2, 4}, {3, 5}, {1, 2}, {3, 4}, {5, 6}};
+    unsigned long long v[W];
+#pragma unroll
+    for (int k = 0; k < W; ++k) v[k] = k < n ? ((unsigned long long)__float_as_uint(raw[k].w) << 3) | k : ~0ull;
+#pragma unroll
+    for (int q = 0; q < (W == 4 ? N4 : N8); ++q) {
+        const unsigned long long lo = min(v[net[q][0]], v[net[q][1]]);
+        const unsigned long long hi = max(v[net[q][0]], v[net[q][1]]);
+        v[net[q][0]] = lo;
+        v[net[q][1]] = hi;
+    }
+#pragma unroll
+    for (int k = 0; k < W; ++k)
+        if (k < n) {
+            b[k] = (int)(v[k] >> 3);
+            e[k] = raw[v[k] & 7];
+        }
 }
 
 /* Orders each cell's beads by index (the order a one-thread FillGrid sweep
    would store them in) and drops the ones beyond the cell capacity, like the
-   `old < GRID_TAIL_SIZE` test of kernel.cl:503. */
-__global__ void k_cell_sort(const RebuildArgs R, int ncells) {
+   `old < GRID_TAIL_SIZE` test of kernel.cl:503.  One thread per cell: cells
+   hold about one bead, and a warp's cells are one run of both arrays (counting
+   each bead's rank with the bead's own thread reads its cell at random: 188 us
+   against 52 on the 4M-bead mat). */
+__global__ void k_cell_sort(const __grid_constant__ RebuildArgs R, int ncells) {
     FN_GATED(R.gate);
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= ncells) return;
     const int n = R.cell_count[c];
-    if (n <= 1) return;
-    int* b = R.cell_beads + R.cell_start[c];
+    if (n == 0) return;
+    const int start = R.cell_start[c];
+    const float4* raw = R.cell_raw + start;
+    int* b = R.cell_beads + start;
+    float4* e = R.cell_pos + start;
+    if (n == 1) {
+        const float4 v = raw[0];
+        b[0] = __float_as_int(v.w);
+        e[0] = v;
+        return;
+    }
+    if (n <= 4 && n <= R.cell_cap) {
+        cell_sort_small<4>(raw, n, b, e);
+        return;
+    }
     if (n <= 8 && n <= R.cell_cap) {
-        /* the common case (about one bead per cell): sorted in registers by
-           Batcher's 8-input network, absent slots holding INT_MAX */
-        int v[8];
-#pragma unroll
-        for (int k = 0; k < 8; ++k) v[k] = k < n ? b[k] : INT_MAX;
-        constexpr int net[19][2] = {{0, 1}, {2, 3}, {4, 5}, {6, 7}, {0, 2}, {1, 3}, {4, 6},
-                                    {5, 7}, {1, 2}, {5, 6}, {0, 4}, {1, 5}, {2, 6}, {3, 7},
-                                    {2, 4}, {3, 5}, {1, 2}, {3, 4}, {5, 6}};
-#pragma unroll
-        for (int q = 0; q < 19; ++q) {
-            const int lo = min(v[net[q][0]], v[net[q][1]]);
-            const int hi = max(v[net[q][0]], v[net[q][1]]);
-            v[net[q][0]] = lo;
-            v[net[q][1]] = hi;
-        }
-#pragma unroll
-        for (int k = 0; k < 8; ++k)
-            if (k < n) b[k] = v[k];
+        cell_sort_small<8>(raw, n, b, e);
         return;
     }
     /* selection of the first min(n, cap) positions: ascending order there,
        O(cap * n) even for an overfull cell */
+    for (int k = 0; k < n; ++k) e[k] = raw[k];
     const int keep = n < R.cell_cap ? n : R.cell_cap;
     for (int k = 0; k < keep; ++k) {
         int best = k;
         for (int m = k + 1; m < n; ++m)
-            if (b[m] < b[best]) best = m;
-        const int v = b[best];
-        b[best] = b[k];
-        b[k] = v;
+            if (__float_as_int(e[m].w) < __float_as_int(e[best].w)) best = m;
+        const float4 v = e[best];
+        e[best] = e[k];
+        e[k] = v;
     }
+    for (int k = 0; k < n; ++k) b[k] = __float_as_int(e[k].w);
     if (n > R.cell_cap) {
         for (int k = R.cell_cap; k < n; ++k) R.cell_of[b[k]] = -1;
         atomicAdd(R.counters + FN_CNT_CELL_OVERFLOW, (unsigned long long)(n - R.cell_cap));
@@ -1370,11 +1399,9 @@ __global__ void k_cell_sort(const RebuildArgs R, int ncells) {
    image) squared distance is known: exclusion of bonded neighbours, then the
    listing radius of the pair kind (the cut-off, widened by the Verlet skin in
    displacement-triggered mode; radius + skin radius for hs pairs). */
-__device__ __forceinline__ bool list_accept(const FnNet& N, const FnPair* __restrict__ pairs,
-                                            double length, double4 pi, int4 bi, double4 pj,
+__device__ __forceinline__ bool list_accept(const FnNet& N, int kind, double length, double4 pi, int4 bi, double4 pj,
                                             int4 bj) {
     if (bi.x == bj.x && abs(bi.y - bj.y) <= 1) return false;
-    const int kind = pairs[N.pair_base + getadress(bi.z, bj.z, N.types_num)].kind;
     if (kind == 1 || kind == 3) return length < N.list_cut_sq;
     if (kind == 2 || kind == 4) {
         if (kind == 4 && length < N.list_cut_sq) return true;
@@ -1386,6 +1413,35 @@ __device__ __forceinline__ bool list_accept(const FnNet& N, const FnPair* __rest
         return length < lim * lim;
     }
     return false;
+}
+
+__device__ __forceinline__ bool list_accept(const FnNet& N, const FnPair* __restrict__ pairs,
+                                            double length, double4 pi, int4 bi, double4 pj,
+                                            int4 bj) {
+    return list_accept(N, pairs[N.pair_base + getadress(bi.z, bj.z, N.types_num)].kind, length, pi, bi, pj, bj);
+}
+
+/* BuildContactList's test of the pair i, j in FP64. */
+template <bool UNIFORM>
+__device__ __forceinline__ bool list_pair(const RebuildArgs& R, const FnNet& N, double4 pi, int4 bi, double4 pj,
+                                          int4 bj) {
+    double rx = pi.x - pj.x, ry = pi.y - pj.y, rz = pi.z - pj.z;
+    double length = rx * rx + ry * ry + rz * rz;
+    if (N.list_mi) length = min_image(N, rx, ry, rz, length, N.list_mi);
+    if (!(length < N.list_r2_max)) return false;
+    return UNIFORM ? list_accept(N, R.pair0.kind, length, pi, bi, pj, bj)
+                   : list_accept(N, R.pairs, length, pi, bi, pj, bj);
+}
+
+/* The second test of a near candidate (its index, the sign set when the first
+   test left its distance open): the exclusion of bonded neighbours, and where
+   the distance is open the test in FP64. */
+template <bool UNIFORM>
+__device__ __forceinline__ bool list_second(const RebuildArgs& R, const FnNet& N, int i, int4 bi, int w, int& j) {
+    j = w & 0x7fffffff;
+    const int4 bj = R.binfo[j];
+    if (bi.x == bj.x && abs(bi.y - bj.y) <= 1) return false;
+    return w >= 0 || list_pair<UNIFORM>(R, N, R.pos[i], bi, R.pos[j], bj);
 }
 
 /* Network owning bead i (networks hold consecutive bead ranges). */
@@ -1420,252 +1476,189 @@ __device__ __forceinline__ void scan_run(const RebuildArgs& R, const FnNet& N, i
     }
 }
 
-/* Full per-bead lists over the 27-cell neighbourhood (dz, dy, dx ascending,
-   beads ascending within a cell): the symmetric closure of the reference's
-   half-shell pair set, in a fixed order.  Threads walk the beads in cell
-   order, so neighbouring threads share their candidate cells; the three
-   cells of one (dz, dy) row are one contiguous run of the sorted bead array
-   unless the row wraps or a cell overflows. */
-/* 12 blocks of 128 per SM (at most 40 registers, a few spilled): the scan
-   waits on dependent loads, and the extra resident warps hide more of that
-   latency than the spills cost (measured: 0.355 vs 0.373 ms per 1M-bead
-   rebuild at the 54 registers the compiler picks unbounded; with the single
-   candidate loop, 0.319 vs 0.327 ms at 10 blocks and 48 registers). */
+/* The place of global cell c in its network's grid. */
+__device__ __forceinline__ void cell_coords(const FnNet& N, int c, int& cx, int& cy, int& cz) {
+    const int lc = max(c - N.cell_base, 0);
+    cz = (int)(__umulhi((unsigned)lc, N.div_nxy) >> N.shift_nxy);
+    const int r = lc - cz * N.nxy;
+    cy = (int)(__umulhi((unsigned)r, N.div_nx) >> N.shift_nx);
+    cx = r - cy * N.nx;
+}
+
 __device__ __forceinline__ void list_one_bead(const RebuildArgs& R, const FnNet& N, int i, int c);
 
-/* Runs of consecutive candidates a thread of k_lists keeps in shared memory
-   (a row of three cells is one run unless it wraps or a cell is full). */
-constexpr int kListRuns = 12;
+/* Full per-bead lists over the 27-cell neighbourhood (dz, dy, dx ascending,
+   beads ascending within a cell): the symmetric closure of the reference's
+   half-shell pair set, in a fixed order.  G lanes of a warp work on one bead;
+   the groups walk the beads in cell order, so neighbouring groups share their
+   candidates' cache lines.
+     1. The nine (dz, dy) rows: three cells of a row are one run of the sorted
+        bead array (two where the row wraps in x); the lanes load the rows'
+        cell starts together and a scan over the group numbers the candidates.
+     2. First test: the candidates, G at a time, from their FP32 positions
+        (16 bytes with the index); the near ones are kept in order by a ballot
+        over the group.
+     3. Second test: the near ones, G at a time, in FP64 with the pair law's
+        radius and the exclusion of bonded neighbours; the accepted ones are
+        written in order by a ballot over the group.
+   A bead whose rows may hold an overfull cell, and boxes too small for the
+   first test, go candidate by candidate in FP64 (list_one_bead).
+   A bead's loads are then a handful of dependent rounds instead of one per
+   candidate, which is what small networks wait for. */
+/* A row's candidates: number k < end is entry (k < split ? a : b) + k; shift says
+   how the bead moves for them, two bits per axis (1 down by the box, 2 up),
+   bits 0-1 for the first part in x, 2-3 for the second, 4-5 y, 6-7 z. */
+struct ListRow {
+    int a, b, split, end;
+};
 
-/* Bead i's candidates (cell c) as runs of the sorted bead array, in list
-   order (dz, dy, dx ascending, beads ascending within a cell); false when
-   they take more than kListRuns runs. */
-__device__ __forceinline__ bool list_runs(const RebuildArgs& R, const FnNet& N, int c, int cz, int cy, int cx,
-                                          int2* runs, int& nr) {
-    for (int dz = -1; dz <= 1; ++dz) {
-        int z = cz + dz;
-        if (z < 0 || z >= N.nz) {
-            if (!(N.periodic & 4)) continue;
-            z = z < 0 ? N.nz - 1 : 0;
-        }
-        for (int dy = -1; dy <= 1; ++dy) {
-            int y = cy + dy;
-            if (y < 0 || y >= N.ny) {
-                if (!(N.periodic & 2)) continue;
-                y = y < 0 ? N.ny - 1 : 0;
-            }
-            const int row = N.cell_base + y * N.nx + z * N.nxy;
-            if (cx >= 1 && cx + 1 < N.nx) {
-                const int c0 = row + cx - 1;
-                const int s0 = R.cell_start[c0];
-                const int s3 = R.cell_start[c0 + 3];
-                if (s3 - s0 <= R.cell_cap ||
-                    (R.cell_count[c0] <= R.cell_cap && R.cell_count[c0 + 1] <= R.cell_cap &&
-                     R.cell_count[c0 + 2] <= R.cell_cap)) {
-                    if (s3 > s0) {
-                        if (nr == kListRuns) return false;
-                        runs[nr++] = make_int2(s0, s3 - s0);
-                    }
-                    continue;
-                }
-            }
-            for (int dx = -1; dx <= 1; ++dx) {
-                int x = cx + dx;
-                if (x < 0 || x >= N.nx) {
-                    if (!(N.periodic & 1)) continue;
-                    x = x < 0 ? N.nx - 1 : 0;
-                }
-                const int nc = row + x;
-                int m = R.cell_count[nc];
-                if (m > R.cell_cap) m = R.cell_cap;
-                if (m > 0) {
-                    if (nr == kListRuns) return false;
-                    runs[nr++] = make_int2(R.cell_start[nc], m);
-                }
-            }
-        }
-    }
-    return true;
-}
+/* The near candidates a group keeps between the tests. */
+constexpr int kListNear = 32;
 
-__global__ void __launch_bounds__(128, 12) k_lists(const RebuildArgs R, long long ncells) {
+template <int G, bool UNIFORM>
+__global__ void __launch_bounds__(128, 10) k_lists_group(const __grid_constant__ RebuildArgs R, long long ncells) {
     FN_GATED(R.gate);
-    __shared__ int2 s_runs[128 * kListRuns];
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= R.cell_start[ncells]) return; /* beads placed in the grid */
-    const int i = R.cell_beads[t];
-    const int c = R.cell_of[i];
-    if (c < 0) return; /* beyond its cell's capacity: listed nowhere */
-    const FnNet& N = R.nets[net_of_bead(R.nets, R.n_nets, i)];
-    /* the bead's candidates as runs of the sorted bead array, in list order
-       (dz, dy, dx ascending, beads ascending within a cell) */
-    int2* runs = s_runs + threadIdx.x * kListRuns;
-    int nr = 0;
-    bool spill = false;
-    const int lc = c - N.cell_base;
-    const int cz = lc / N.nxy;
-    const int cy = (lc - cz * N.nxy) / N.nx;
-    const int cx = lc - cz * N.nxy - cy * N.nx;
-    for (int dz = -1; dz <= 1 && !spill; ++dz) {
-        int z = cz + dz;
-        if (z < 0 || z >= N.nz) {
-            if (!(N.periodic & 4)) continue;
-            z = z < 0 ? N.nz - 1 : 0;
-        }
-        for (int dy = -1; dy <= 1 && !spill; ++dy) {
-            int y = cy + dy;
-            if (y < 0 || y >= N.ny) {
-                if (!(N.periodic & 2)) continue;
-                y = y < 0 ? N.ny - 1 : 0;
-            }
-            const int row = N.cell_base + y * N.nx + z * N.nxy;
-            if (cx >= 1 && cx + 1 < N.nx) {
-                const int c0 = row + cx - 1;
-                const int s0 = R.cell_start[c0];
-                const int s3 = R.cell_start[c0 + 3];
-                if (s3 - s0 <= R.cell_cap ||
-                    (R.cell_count[c0] <= R.cell_cap && R.cell_count[c0 + 1] <= R.cell_cap &&
-                     R.cell_count[c0 + 2] <= R.cell_cap)) {
-                    if (s3 > s0) {
-                        if (nr == kListRuns) {
-                            spill = true;
-                            break;
-                        }
-                        runs[nr++] = make_int2(s0, s3 - s0);
-                    }
-                    continue;
-                }
-            }
-            for (int dx = -1; dx <= 1; ++dx) {
-                int x = cx + dx;
-                if (x < 0 || x >= N.nx) {
-                    if (!(N.periodic & 1)) continue;
-                    x = x < 0 ? N.nx - 1 : 0;
-                }
-                const int nc = row + x;
-                int m = R.cell_count[nc];
-                if (m > R.cell_cap) m = R.cell_cap;
-                if (m > 0) {
-                    if (nr == kListRuns) {
-                        spill = true;
-                        break;
-                    }
-                    runs[nr++] = make_int2(R.cell_start[nc], m);
-                }
-            }
-        }
-    }
-    if (spill) { /* more runs than the table holds: the row-by-row scan */
-        list_one_bead(R, N, i, c);
-        return;
-    }
-    /* one loop over all runs, so a warp iterates as often as its busiest lane
-       has candidates, not as often as the sum of each row's busiest lane */
-    const double4 pi = R.pos[i];
-    const int4 bi = R.binfo[i];
-    int* __restrict__ out = R.list + i;
-    int n = 0;
-    int r = 0, q = 0, qe = 0;
-    if (nr > 0) {
-        q = runs[0].x;
-        qe = q + runs[0].y;
-    }
-    while (r < nr) {
-        const int j = R.cell_beads[q];
-        if (j != i) {
-            const double4 pj = R.pos[j];
-            double rx = pi.x - pj.x, ry = pi.y - pj.y, rz = pi.z - pj.z;
-            double length = rx * rx + ry * ry + rz * rz;
-            if (N.list_mi) length = min_image(N, rx, ry, rz, length, N.list_mi);
-            if (length < N.list_r2_max && list_accept(N, R.pairs, length, pi, bi, pj, R.binfo[j])) {
-                if (n < R.list_cap) out[(size_t)n * R.list_stride] = j;
-                ++n;
-            }
-        }
-        if (++q == qe && ++r < nr) {
-            q = runs[r].x;
-            qe = q + runs[r].y;
-        }
-    }
-    if (n > R.list_cap)
-        atomicAdd(R.counters + FN_CNT_LIST_OVERFLOW, (unsigned long long)(n - R.list_cap));
-    R.list_count[i] = n;
-}
-
-/* BuildContactList with G lanes per bead (the same lists as k_lists, entry
-   for entry), for networks too small to hide k_lists' chain of dependent
-   loads with one thread per bead: a bead's candidates are taken G at a time,
-   lane l of its group testing candidate (round x G + l), and the accepted
-   ones are written in candidate order by a ballot over the group.  Blocks
-   of 128 threads, 128 / G beads in cell order. */
-template <int G>
-__global__ void __launch_bounds__(128) k_lists_group(const RebuildArgs R, long long ncells) {
-    FN_GATED(R.gate);
-    constexpr int PER = 128 / G;
-    __shared__ int2 s_runs[PER * kListRuns];
-    __shared__ int s_nr[PER];
+    constexpr int PER = 128 / G, J = (9 + G - 1) / G;
+    __shared__ ListRow s_row[9 * PER];
+    __shared__ unsigned char s_shift[9 * PER];
+    __shared__ int s_near[kListNear * PER];
+    const unsigned full = 0xffffffffu;
     const int lane = threadIdx.x & 31, gl = threadIdx.x % G, grp = threadIdx.x / G;
     const int t = blockIdx.x * PER + grp;
-    int i = -1, c = -1;
+    int i = -1, c = 0;
+    float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
     if (t < R.cell_start[ncells]) { /* beads placed in the grid */
-        i = R.cell_beads[t];
+        o = R.cell_pos[t];
+        i = __float_as_int(o.w);
         c = R.cell_of[i];
         if (c < 0) i = -1; /* beyond its cell's capacity: listed nowhere */
     }
-    const FnNet& N = R.nets[i >= 0 ? net_of_bead(R.nets, R.n_nets, i) : 0];
-    int2* runs = s_runs + grp * kListRuns;
-    if (gl == 0) {
-        int nr = 0;
-        if (i >= 0) {
-            const int lc = c - N.cell_base;
-            const int cz = lc / N.nxy;
-            const int cy = (lc - cz * N.nxy) / N.nx;
-            const int cx = lc - cz * N.nxy - cy * N.nx;
-            if (!list_runs(R, N, c, cz, cy, cx, runs, nr)) nr = -1; /* row by row, below */
-        }
-        s_nr[grp] = nr;
-    }
-    __syncwarp(); /* a group's lanes share a warp */
-    const int nr = s_nr[grp];
+    const FnNet& N = UNIFORM ? R.net0 : R.nets[i >= 0 ? net_of_bead(R.nets, R.n_nets, i) : 0];
+    const float r2 = N.list_out_r2;
+    bool plain = !(r2 >= 0.0f); /* no first test */
+    ListRow* rows = s_row + 9 * grp;
+    unsigned char* shifts = s_shift + 9 * grp;
+    int* near = s_near + kListNear * grp;
     int total = 0;
-    for (int r = 0; r < nr; ++r) total += runs[r].y;
-    const int rounds = __reduce_max_sync(0xffffffffu, (total + G - 1) / G);
-    double4 pi = make_double4(0.0, 0.0, 0.0, 0.0);
-    int4 bi = make_int4(0, 0, 0, 0);
-    if (nr > 0) {
-        pi = R.pos[i];
-        bi = R.binfo[i];
-    }
-    const unsigned gmask = G == 32 ? 0xffffffffu : (((1u << G) - 1u) << (lane & ~(G - 1)));
-    const unsigned below = (1u << lane) - 1u;
-    int* __restrict__ out = R.list + (i >= 0 ? i : 0);
-    int n = 0;
-    int r = 0, off = gl; /* this lane's candidate: offset off in run r */
-    while (r < nr && off >= runs[r].y) off -= runs[r++].y;
-    for (int k = 0; k < rounds; ++k) {
-        bool acc = false;
-        int j = -1;
-        if (r < nr) {
-            j = R.cell_beads[runs[r].x + off];
-            if (j != i) {
-                const double4 pj = R.pos[j];
-                double rx = pi.x - pj.x, ry = pi.y - pj.y, rz = pi.z - pj.z;
-                double length = rx * rx + ry * ry + rz * rz;
-                if (N.list_mi) length = min_image(N, rx, ry, rz, length, N.list_mi);
-                acc = length < N.list_r2_max && list_accept(N, R.pairs, length, pi, bi, pj, R.binfo[j]);
+    bool moved = false; /* some row lies beyond a periodic side */
+    {
+        int cx, cy, cz;
+        cell_coords(N, c, cx, cy, cz);
+        const int xa = max(cx - 1, 0), xb = min(cx + 2, N.nx);
+        const bool wl = cx == 0 && (N.periodic & 1), wr = cx + 1 == N.nx && (N.periodic & 1);
+#pragma unroll
+        for (int q = 0; q < J; ++q) {
+            const int k = q * G + gl;
+            int a0 = 0, na = 0, b0 = 0, nb = 0, shift = 0;
+            if (k < 9 && i >= 0) {
+                int z = cz + k / 3 - 1, y = cy + k % 3 - 1;
+                bool ok = true;
+                /* a cell below the grid lies at the far side: the bead moves up */
+                if (z < 0 || z >= N.nz) {
+                    ok = N.periodic & 4;
+                    shift |= z < 0 ? 128 : 64;
+                    z = z < 0 ? N.nz - 1 : 0;
+                }
+                if (y < 0 || y >= N.ny) {
+                    ok = ok && (N.periodic & 2);
+                    shift |= y < 0 ? 32 : 16;
+                    y = y < 0 ? N.ny - 1 : 0;
+                }
+                if (ok) {
+                    const int* row = R.cell_start + (N.cell_base + y * N.nx + z * N.nxy);
+                    a0 = row[xa];
+                    na = row[xb] - a0;
+                    if (wl) { /* the cell beyond the side comes first */
+                        b0 = a0;
+                        nb = na;
+                        a0 = row[N.nx - 1];
+                        na = row[N.nx] - a0;
+                        shift |= 2;
+                    } else if (wr) {
+                        b0 = row[0];
+                        nb = row[1] - b0;
+                        shift |= 4;
+                    }
+                    if (na > R.cell_cap || nb > R.cell_cap) plain = true;
+                }
             }
+            /* number the candidates: inclusive scan over the group's lanes */
+            int e = na + nb;
+#pragma unroll
+            for (int d = 1; d < G; d <<= 1) {
+                const int v = __shfl_up_sync(full, e, d, G);
+                if (gl >= d) e += v;
+            }
+            const int first = total + e - na - nb;
+            if (k < 9) {
+                rows[k] = ListRow{a0 - first, b0 - first - na, first + na, first + na + nb};
+                shifts[k] = (unsigned char)shift;
+            }
+            moved |= shift != 0;
+            total += __shfl_sync(full, e, G - 1, G);
         }
-        const unsigned mine = __ballot_sync(0xffffffffu, acc) & gmask;
-        if (acc) {
-            const int pos = n + __popc(mine & below);
-            if (pos < R.list_cap) out[(size_t)pos * R.list_stride] = j;
-        }
-        n += __popc(mine);
-        off += G;
-        while (r < nr && off >= runs[r].y) off -= runs[r++].y;
     }
+    const unsigned gmask = G == 32 ? full : (((1u << G) - 1u) << (lane & ~(G - 1)));
+    const unsigned below = (1u << lane) - 1u;
+    plain = (__ballot_sync(full, plain) & gmask) != 0;
+    moved = __any_sync(full, moved);
+    if (plain || i < 0) total = 0;
+    __syncwarp();
+    int4 bi = make_int4(0, 0, 0, 0);
+    if (total > 0) bi = R.binfo[i];
+    const float in_r2 = N.list_in_r2;
+    int* __restrict__ out = R.list + (i >= 0 ? i : 0);
+    int n = 0, m = 0;
+    /* second test of the m near candidates */
+    auto flush = [&]() {
+        __syncwarp();
+        const int most = __reduce_max_sync(full, m);
+        for (int k0 = 0; k0 < most; k0 += G) {
+            const int k = k0 + gl;
+            bool acc = false;
+            int j = -1;
+            if (k < m) acc = list_second<UNIFORM>(R, N, i, bi, near[k], j);
+            const unsigned mine = __ballot_sync(full, acc) & gmask;
+            if (acc) {
+                const int at = n + __popc(mine & below);
+                if (at < R.list_cap) out[(size_t)at * R.list_stride] = j;
+            }
+            n += __popc(mine);
+        }
+        m = 0;
+        __syncwarp();
+    };
+    const int most = __reduce_max_sync(full, total);
+    ListRow u = rows[0];
+    int r = 0;
+    for (int k0 = 0; k0 < most; k0 += G) {
+        const int k = k0 + gl;
+        bool hit = false;
+        int j = -1;
+        if (k < total) {
+            while (k >= u.end) u = rows[++r];
+            const float4 e = R.cell_pos[(k < u.split ? u.a : u.b) + k];
+            j = __float_as_int(e.w);
+            float dx = o.x - e.x, dy = o.y - e.y, dz = o.z - e.z;
+            if (moved) {
+                const int sh = shifts[r], sx = k < u.split ? sh : sh >> 2;
+                const float bx = (float)N.box[0], by = (float)N.box[1], bz = (float)N.box[2];
+                dx += sx & 1 ? -bx : sx & 2 ? bx : 0.0f;
+                dy += sh & 16 ? -by : sh & 32 ? by : 0.0f;
+                dz += sh & 64 ? -bz : sh & 128 ? bz : 0.0f;
+            }
+            const float d2 = __fmaf_rn(dx, dx, __fmaf_rn(dy, dy, dz * dz));
+            hit = d2 <= r2 && j != i;
+            if (!(d2 <= in_r2)) j |= (int)0x80000000;
+        }
+        const unsigned mine = __ballot_sync(full, hit) & gmask;
+        if (hit) near[m + __popc(mine & below)] = j;
+        m += __popc(mine);
+        if (__any_sync(full, m > kListNear - G)) flush();
+    }
+    flush();
     if (gl == 0 && i >= 0) {
-        if (nr < 0) {
+        if (plain) {
             list_one_bead(R, N, i, c);
         } else {
             if (n > R.list_cap)
@@ -1673,6 +1666,136 @@ __global__ void __launch_bounds__(128) k_lists_group(const RebuildArgs R, long l
             R.list_count[i] = n;
         }
     }
+}
+
+/* Near candidates a thread of k_lists keeps between its two tests. */
+constexpr int kListKeep = 24;
+
+/* The same lists with one thread per bead, for networks large enough to hide
+   one thread's loads: fewer instructions per bead (no scan, no ballots).
+   Bound by instruction issue (about 3,300 per warp, 60 % of the slots) and
+   load latency.  The FP32 test from 16 bytes per candidate, with FP64 only
+   where it cannot decide, took the rebuild of the 1M-bead tensile network
+   from 313 to 211 us and that of the 4M-bead mat from 1,340 to 943 us. */
+template <bool UNIFORM>
+__global__ void __launch_bounds__(128, 8) k_lists(const __grid_constant__ RebuildArgs R, long long ncells) {
+    FN_GATED(R.gate);
+    __shared__ int s_first[9 * 128];
+    __shared__ unsigned char s_len[9 * 128];
+    __shared__ int s_near[kListKeep * 128];
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= R.cell_start[ncells]) return; /* beads placed in the grid */
+    const float4 o = R.cell_pos[t];
+    const int i = __float_as_int(o.w);
+    const int c = R.cell_of[i];
+    if (c < 0) return; /* beyond its cell's capacity: listed nowhere */
+    const FnNet& N = UNIFORM ? R.net0 : R.nets[net_of_bead(R.nets, R.n_nets, i)];
+    const float out_r2 = N.list_out_r2, in_r2 = N.list_in_r2;
+    int* first = s_first + threadIdx.x;
+    unsigned char* len = s_len + threadIdx.x;
+    int* near = s_near + threadIdx.x;
+    int cx, cy, cz;
+    cell_coords(N, c, cx, cy, cz);
+    const int cap = min(R.cell_cap, 255);
+    /* the nine rows (dz, dy ascending): the row's cells in place are one run
+       of the sorted arrays; all cell starts are loaded together */
+    const int xa = max(cx - 1, 0), xb = min(cx + 2, N.nx);
+    const int zlo = cz > 0 ? -N.nxy : N.periodic & 4 ? (N.nz - 1) * N.nxy : INT_MIN;
+    const int zhi = cz + 1 < N.nz ? N.nxy : N.periodic & 4 ? -cz * N.nxy : INT_MIN;
+    const int ylo = cy > 0 ? -N.nx : N.periodic & 2 ? (N.ny - 1) * N.nx : INT_MIN;
+    const int yhi = cy + 1 < N.ny ? N.nx : N.periodic & 2 ? -cy * N.nx : INT_MIN;
+    bool plain = !(out_r2 >= 0.0f);
+    const int* own = R.cell_start + (c - cx);
+    {
+        int s0[9], s1[9];
+#pragma unroll
+        for (int k = 0; k < 9; ++k) {
+            const int dz = k < 3 ? zlo : k < 6 ? 0 : zhi, dy = k % 3 == 0 ? ylo : k % 3 == 1 ? 0 : yhi;
+            const bool ok = dz != INT_MIN && dy != INT_MIN;
+            const int* row = own + (ok ? dz + dy : 0);
+            s0[k] = row[xa];
+            s1[k] = ok ? row[xb] : s0[k];
+        }
+#pragma unroll
+        for (int k = 0; k < 9; ++k) {
+            plain = plain || s1[k] - s0[k] > cap;
+            first[128 * k] = s0[k];
+            len[128 * k] = (unsigned char)(s1[k] - s0[k]);
+        }
+    }
+    /* beyond a periodic side in x, one more cell of each row, before or after
+       the others */
+    const bool wl = cx == 0 && (N.periodic & 1), wr = cx + 1 == N.nx && (N.periodic & 1);
+    const bool moved = wl || wr || (cz == 0 || cz + 1 == N.nz) || (cy == 0 || cy + 1 == N.ny);
+    const int4 bi = R.binfo[i];
+    int* __restrict__ out = R.list + i;
+    int n = 0, m = 0;
+    /* second test of the near candidates */
+    auto flush = [&]() {
+        for (int k = 0; k < m; ++k) {
+            int j;
+            if (list_second<UNIFORM>(R, N, i, bi, near[128 * k], j)) { /* i itself is excluded, as a bonded neighbour */
+                if (n < R.list_cap) out[(size_t)n * R.list_stride] = j;
+                ++n;
+            }
+        }
+        m = 0;
+    };
+    for (int k = 0; k < 9 && !plain; ++k) {
+        float ox = o.x, oy = o.y, oz = o.z;
+        int q = first[128 * k], left = len[128 * k];
+        int q2 = 0, left2 = 0;
+        if (moved) {
+            /* cells below the grid lie at the far side: the bead moves up */
+            const int dz = k < 3 ? zlo : k < 6 ? 0 : zhi, dy = k % 3 == 0 ? ylo : k % 3 == 1 ? 0 : yhi;
+            if (k < 3 && cz == 0) oz += (float)N.box[2];
+            if (k >= 6 && cz + 1 == N.nz) oz -= (float)N.box[2];
+            if (k % 3 == 0 && cy == 0) oy += (float)N.box[1];
+            if (k % 3 == 2 && cy + 1 == N.ny) oy -= (float)N.box[1];
+            if ((wl || wr) && dz != INT_MIN && dy != INT_MIN) {
+                const int* w = own + dz + dy + (wl ? N.nx - 1 : 0);
+                q2 = w[0];
+                left2 = w[1] - q2;
+                if (left2 > cap) plain = true;
+                if (wl) { /* first */
+                    int v = q;
+                    q = q2;
+                    q2 = v;
+                    v = left;
+                    left = left2;
+                    left2 = v;
+                    ox += (float)N.box[0];
+                }
+            }
+        }
+        for (int part = 0; part < 2; ++part) {
+            while (left > 0) {
+                if (m + left > kListKeep) flush();
+                const int stop = q + min(left, kListKeep);
+                left -= stop - q;
+#pragma unroll 2
+                for (; q < stop; ++q) {
+                    const float4 v = R.cell_pos[q];
+                    const float dx = ox - v.x, dy = oy - v.y, dz = oz - v.z;
+                    const float d2 = __fmaf_rn(dx, dx, __fmaf_rn(dy, dy, dz * dz));
+                    if (d2 <= out_r2) near[128 * m++] = __float_as_int(v.w) | (d2 <= in_r2 ? 0 : (int)0x80000000);
+                }
+            }
+            if (left2 == 0) break;
+            q = q2;
+            left = left2;
+            left2 = 0;
+            ox = wl ? o.x : o.x - (float)N.box[0];
+        }
+    }
+    if (plain) {
+        list_one_bead(R, N, i, c); /* candidate by candidate in FP64 */
+        return;
+    }
+    flush();
+    if (n > R.list_cap)
+        atomicAdd(R.counters + FN_CNT_LIST_OVERFLOW, (unsigned long long)(n - R.list_cap));
+    R.list_count[i] = n;
 }
 
 /* Bead i's full list, reading its candidates from global memory (k_lists,
@@ -2295,6 +2418,23 @@ cudaError_t launch_exclusive_scan(const int* in, long long n, int* out, int* blo
     return cudaGetLastError();
 }
 
+/* Largest context whose bead-by-bead build takes four lanes per bead: below
+   it one thread per bead leaves the SMs waiting for its loads (whole rebuild,
+   four lanes against one: 10k beads 38 against 42 us, 100k dense 60 against
+   91, 111k tensile 68 against 66), above it the instructions of the scan and
+   the ballots count (300k tensile 111 against 90, 1M 320 against 211). */
+constexpr int kGroupedBeads = 200000;
+
+/* every bead may sit in the grid; groups past the grid total do nothing */
+template <int G>
+static void launch_lists_group(const RebuildArgs& R, int nb, long long ncells, cudaStream_t s) {
+    constexpr int PER = 128 / G;
+    if (R.uniform)
+        k_lists_group<G, true><<<(nb + PER - 1) / PER, 128, 0, s>>>(R, ncells);
+    else
+        k_lists_group<G, false><<<(nb + PER - 1) / PER, 128, 0, s>>>(R, ncells);
+}
+
 cudaError_t launch_rebuild(const RebuildArgs& R, int ntiles, int block, int nb, long long ncells,
                            int* scan_block_sums, cudaStream_t s) {
     cudaError_t e;
@@ -2316,10 +2456,14 @@ cudaError_t launch_rebuild(const RebuildArgs& R, int ntiles, int block, int nb, 
     if (R.bricks) {
         if (R.nbricks > 0) k_lists_brick<<<R.nbricks, kBrickThreads, 0, s>>>(R, R.bricks);
     } else if (nb > 0 && R.list_lanes == 8) {
-        k_lists_group<8><<<(nb + 15) / 16, 128, 0, s>>>(R, ncells);
+        launch_lists_group<8>(R, nb, ncells, s);
+    } else if (nb > 0 && nb <= kGroupedBeads) {
+        launch_lists_group<4>(R, nb, ncells, s);
     } else if (nb > 0) {
-        /* every bead may sit in the grid; threads past the grid total return */
-        k_lists<<<(nb + 127) / 128, 128, 0, s>>>(R, ncells);
+        if (R.uniform)
+            k_lists<true><<<(nb + 127) / 128, 128, 0, s>>>(R, ncells);
+        else
+            k_lists<false><<<(nb + 127) / 128, 128, 0, s>>>(R, ncells);
     }
     /* the staged step kernel's copy, one block per tile (tiles are at most
        block - 4 beads wide) */

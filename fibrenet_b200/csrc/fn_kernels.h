@@ -203,6 +203,10 @@ struct RebuildArgs {
     int* cell_fill;
     int* cell_start; /* ncells + 1 */
     int* cell_beads;
+    /* FP32 position and index (bits) of each bead in the grid: by cell in the
+       order of arrival, and like cell_beads */
+    float4* cell_raw;
+    float4* cell_pos;
     int* list_count;
     int* list;
     int list_stride;
@@ -215,13 +219,17 @@ struct RebuildArgs {
        the per-bead list build) */
     const int4* bricks;
     int nbricks;
-    /* lanes per bead of the grouped list build (k_lists_group), 0: one
-       thread per bead (k_lists) */
+    /* 8: the list build by groups of 8 lanes per bead; 0: bead by bead (one
+       thread or, in small contexts, four lanes each) */
     int list_lanes;
     /* tile-compacted copy of the list for the staged step kernel (null: none) */
     int* csr;
     long long csr_region;
     int* tile_items;
+    /* one network with one pair law for all bead types: both by value */
+    int uniform;
+    FnNet net0;
+    FnPair pair0;
 };
 
 struct ObserveArgs {
@@ -289,7 +297,7 @@ struct UpRaw {
 struct UpCheck {
     int bad_bead, bad_spring, bad_angle; /* first offending index, INT_MAX if none */
     int not_runs;                        /* springs not joining consecutive beads */
-    unsigned long long rmax, smax, gmin; /* order-preserving keys of the radius extremes */
+    unsigned long long rmax, smax, gmin, rmin; /* order-preserving keys of the radius extremes */
 };
 
 cudaError_t launch_upload_checks(const UpNet* nets, int n_nets, const UpRaw& R, UpCheck* out, int nb, int ns, int na,

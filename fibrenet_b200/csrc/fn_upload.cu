@@ -56,7 +56,7 @@ __device__ __forceinline__ unsigned long long dkey(double x) {
    the float-rounded radius. */
 __global__ void __launch_bounds__(256) k_up_beads_check(const UpNet* __restrict__ nets, int n_nets, UpRaw R,
                                                         UpCheck* out, int nb) {
-    __shared__ unsigned long long s_max_r[8], s_max_s[8], s_min_g[8];
+    __shared__ unsigned long long s_max_r[8], s_max_s[8], s_min_g[8], s_min_r[8];
     __shared__ int s_net0, s_net1;
     const int u = blockIdx.x * blockDim.x + threadIdx.x;
     const int first = blockIdx.x * blockDim.x;
@@ -66,7 +66,7 @@ __global__ void __launch_bounds__(256) k_up_beads_check(const UpNet* __restrict_
         s_net1 = up_net(nets, n_nets, last, 0);
     }
     __syncthreads();
-    unsigned long long kr = 0, ks = 0, kg = ~0ull;
+    unsigned long long kr = 0, ks = 0, kg = ~0ull, km = ~0ull;
     int k = s_net0;
     if (u < nb) {
         k = s_net0 == s_net1 ? s_net0 : up_net(nets, n_nets, u, 0);
@@ -77,7 +77,7 @@ __global__ void __launch_bounds__(256) k_up_beads_check(const UpNet* __restrict_
         if (t < 0 || t >= N.n_types || !(mass >= 0.0)) atomicMin(&out[k].bad_bead, i);
         const float rad = (float)R.radius[u];
         const float skin = (float)((double)rad + N.skin_ratio);
-        kr = dkey((double)rad);
+        kr = km = dkey((double)rad);
         ks = dkey((double)skin);
         kg = dkey((double)skin - (double)rad);
     }
@@ -87,6 +87,7 @@ __global__ void __launch_bounds__(256) k_up_beads_check(const UpNet* __restrict_
             atomicMax(&out[k].rmax, kr);
             atomicMax(&out[k].smax, ks);
             atomicMin(&out[k].gmin, kg);
+            atomicMin(&out[k].rmin, km);
         }
         return;
     }
@@ -95,12 +96,14 @@ __global__ void __launch_bounds__(256) k_up_beads_check(const UpNet* __restrict_
         kr = max(kr, __shfl_xor_sync(0xffffffffu, kr, o));
         ks = max(ks, __shfl_xor_sync(0xffffffffu, ks, o));
         kg = min(kg, __shfl_xor_sync(0xffffffffu, kg, o));
+        km = min(km, __shfl_xor_sync(0xffffffffu, km, o));
     }
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (lane == 0) {
         s_max_r[w] = kr;
         s_max_s[w] = ks;
         s_min_g[w] = kg;
+        s_min_r[w] = km;
     }
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -109,10 +112,12 @@ __global__ void __launch_bounds__(256) k_up_beads_check(const UpNet* __restrict_
             kr = max(kr, s_max_r[q]);
             ks = max(ks, s_max_s[q]);
             kg = min(kg, s_min_g[q]);
+            km = min(km, s_min_r[q]);
         }
         atomicMax(&out[k].rmax, kr);
         atomicMax(&out[k].smax, ks);
         atomicMin(&out[k].gmin, kg);
+        atomicMin(&out[k].rmin, km);
     }
 }
 

@@ -449,8 +449,8 @@ class Simulation:
     LIST_BUILDS = ("beads", "bricks", "groups")
 
     def set_list_build(self, mode) -> None:
-        """How contact lists are built: "beads" (one thread per bead, the
-        default; also False / 0), "bricks" (cells staged in shared memory;
+        """How contact lists are built: "beads" (bead by bead, the default;
+        also False / 0), "bricks" (cells staged in shared memory;
         also True / 1) or "groups" (8 lanes per bead; also 2)."""
         m = self.LIST_BUILDS.index(mode) if isinstance(mode, str) else int(mode)
         self._check(self.lib.fn_set_list_build(self.h, m))

@@ -364,8 +364,8 @@ FN_API int fn_device_view(fn_ctx* ctx, int field, fn_view* out);
 FN_API int fn_autotune(fn_ctx* ctx, int steps_per_trial);
 
 /* How contact lists are built (ResetGrid .. BuildContactList,
-   kernel.cl:487-789): 0 (the default) one thread per bead reading its
-   candidates from global memory; 1 by bricks of 8 x 4 x 4 grid cells whose
+   kernel.cl:487-789): 0 (the default) bead by bead, one thread per bead or, in
+   contexts of at most 200,000 beads, four lanes; 1 by bricks of 8 x 4 x 4 grid cells whose
    beads and neighbouring beads are staged in shared memory; 2 by groups of 8
    lanes per bead (more threads in flight for small networks).  All give the
    same lists, entry for entry; fn_autotune keeps the fastest. */

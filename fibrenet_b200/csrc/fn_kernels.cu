@@ -34,6 +34,16 @@
 
 namespace fn {
 
+/* Programmatic dependent launch (launch_next): a kernel of the step sequence
+   waits on the device for the kernel before it, all of its blocks and writes,
+   before it touches anything that kernels write, and says when the next one's
+   blocks may be placed.  The launch itself, 1.5 us and more between dependent
+   kernels of a stream, then runs beside the kernel before it.  Every thread of
+   every kernel that launch_next starts must wait, whatever it does next: one
+   that ended without waiting would let its successor run beside its
+   predecessor. */
+__device__ __forceinline__ void await_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void let_next_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 __device__ __forceinline__ int spring_pts(double ax, double ay, double az, double bx, double by,
                                           double bz, float4 par, int type, double& fx, double& fy,
@@ -334,6 +344,9 @@ enum { FN_STEP_SPRINGS = 1, FN_STEP_ANGLES = 2, FN_STEP_CONTACTS = 4, FN_STEP_DR
 template <bool DAMP>
 __device__ __forceinline__ void kick_drift(const StepArgs& A, const FnNet& N, int i, double4 p, double Fx, double Fy,
                                            double Fz, bool do_drift, bool store_v) {
+    /* late: the next step's blocks take shared memory and slots from this one's
+       (60k beads: 19.1 us per step, 20.2 with this at the kernel's start) */
+    let_next_start();
     /* loaded before the finiteness test: behind its branch these loads, and
        with them every load of the kernel that reaches DRAM, take twice as
        long (1M-bead tensile step 204 us against 108, the same sectors, hits
@@ -394,6 +407,7 @@ __device__ __forceinline__ void finish_bead(const StepArgs& A, const FnNet& N, i
 
 template <bool DAMP>
 __global__ void __launch_bounds__(512) k_step(const __grid_constant__ StepArgs A, int flags) {
+    await_previous();
     const FnTile t = A.tiles[blockIdx.x];
     const int i = t.begin + (int)threadIdx.x;
     if (i >= t.end) return;
@@ -466,6 +480,7 @@ __global__ void __launch_bounds__(512) k_step(const __grid_constant__ StepArgs A
    the same order as k_step, so the result is bit-identical to k_step. */
 template <bool DAMP, bool UNIFORM>
 __global__ void __launch_bounds__(512) k_step_tiled(const __grid_constant__ StepArgs A, int flags) {
+    await_previous();
     extern __shared__ double smem[];
     const int t = blockIdx.x;
     const FnTile tile = A.tiles[t];
@@ -628,14 +643,19 @@ __global__ void __launch_bounds__(kChainMaxBlock, 4) k_step_chain(const __grid_c
     double* s_ang = reinterpret_cast<double*>(smem_raw + L.ang);
     unsigned char* s_ok = smem_raw + L.ok;
 
+    /* tiles and flags are written by no kernel of the step sequence; loading the
+       bonds' records here too gains 2 % on 480 beads and costs 1.5 % on the
+       large networks (registers) */
+    const bool mine = tid < n + 4 && i >= 0 && i < A.nb;
     unsigned fl = 0, st0 = 0;
+    if (mine) fl = A.ch_flags[i];
+    await_previous();
     double x = 0.0, y = 0.0, z = 0.0;
-    if (tid < n + 4 && i >= 0 && i < A.nb) {
+    if (mine) {
         const double4 q = A.img_in[i];
         x = q.x;
         y = q.y;
         z = q.z;
-        fl = A.ch_flags[i];
         st0 = A.ch_status[i];
     }
     s_img[3 * tid] = x;
@@ -653,12 +673,12 @@ __global__ void __launch_bounds__(kChainMaxBlock, 4) k_step_chain(const __grid_c
         z -= s_img[3 * tid + 5];
         root_and_inverse(x * x + y * y + z * z, l, il);
         if ((fl & FN_CH_SPRING) && (st0 & 1) && !(fl & FN_CH_SP_INERT)) {
-            const float4 par = A.ch_sp[i];
-            double factor = (double)par.x - l;
-            if ((fl & FN_CH_SP_FL) && fabs(-(double)par.z * factor * il) > (double)par.w) {
+            const float4 sp = A.ch_sp[i];
+            double factor = (double)sp.x - l;
+            if ((fl & FN_CH_SP_FL) && fabs(-(double)sp.z * factor * il) > (double)sp.w) {
                 st &= ~1u; /* breaks: no force from this step on (kernel.cl:391-397) */
             } else if (!FORCES_ONLY || (flags & FN_STEP_SPRINGS)) {
-                factor *= (double)par.y;
+                factor *= (double)sp.y;
                 gx = x * il * factor;
                 gy = y * il * factor;
                 gz = z * il * factor;
@@ -940,6 +960,7 @@ __device__ __forceinline__ void gather_partners(const StepArgs& A, const int* __
    Tiles with more contact items than `chunk` take them in rounds. */
 template <bool DAMP, bool DRIFT, bool STORE_V>
 __global__ void __launch_bounds__(kChainMaxBlock) k_step_staged(const StepArgs A) {
+    await_previous();
     extern __shared__ __align__(128) unsigned char sm[];
     const StagedSmem L = staged_smem_layout(blockDim.x, A.chunk);
     const FnTile tile = A.tiles[blockIdx.x];
@@ -1189,6 +1210,8 @@ __global__ void __launch_bounds__(kChainMaxBlock) k_step_staged(const StepArgs A
 
 template <bool STORE_V>
 __global__ void __launch_bounds__(512) k_drift(const StepArgs A) {
+    await_previous();
+    let_next_start();
     const FnTile t = A.tiles[blockIdx.x];
     const int i = t.begin + (int)threadIdx.x;
     if (i >= t.end) return;
@@ -1282,6 +1305,8 @@ __global__ void k_reset_energy(float4* force, float4* vel, float4* vold, int n) 
     return
 
 __global__ void k_fill_int(int* p, long long n, int v, const int* gate) {
+    await_previous();
+    let_next_start();
     FN_GATED(gate);
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
          i += (long long)gridDim.x * blockDim.x)
@@ -1289,6 +1314,8 @@ __global__ void k_fill_int(int* p, long long n, int v, const int* gate) {
 }
 
 __global__ void k_cells(const RebuildArgs R) {
+    await_previous();
+    let_next_start();
     FN_GATED(R.gate);
     const FnTile t = R.tiles[blockIdx.x];
     const int i = t.begin + (int)threadIdx.x;
@@ -1306,11 +1333,14 @@ __global__ void k_cells(const RebuildArgs R) {
     }
     R.cell_of[i] = cell;
     R.list_count[i] = 0; /* k_lists counts only the beads it lists */
+    if (R.ref) R.ref[i] = R.img[i];
 }
 
 /* FillGrid's slot of each bead in its cell: the bead as the list build's first
    test reads it, 16 bytes with its position rounded to FP32 and its index. */
 __global__ void k_scatter(const __grid_constant__ RebuildArgs R, int nb) {
+    await_previous();
+    let_next_start();
     FN_GATED(R.gate);
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= nb) return;
@@ -1353,6 +1383,8 @@ __device__ __forceinline__ void cell_sort_small(const float4* raw, int n, int* b
    each bead's rank with the bead's own thread reads its cell at random: 188 us
    against 52 on the 4M-bead mat). */
 __global__ void k_cell_sort(const __grid_constant__ RebuildArgs R, int ncells) {
+    await_previous();
+    let_next_start();
     FN_GATED(R.gate);
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= ncells) return;
@@ -1517,6 +1549,7 @@ constexpr int kListNear = 32;
 
 template <int G, bool UNIFORM>
 __global__ void __launch_bounds__(128, 10) k_lists_group(const __grid_constant__ RebuildArgs R, long long ncells) {
+    await_previous();
     FN_GATED(R.gate);
     constexpr int PER = 128 / G, J = (9 + G - 1) / G;
     __shared__ ListRow s_row[9 * PER];
@@ -1679,6 +1712,7 @@ constexpr int kListKeep = 24;
    from 313 to 211 us and that of the 4M-bead mat from 1,340 to 943 us. */
 template <bool UNIFORM>
 __global__ void __launch_bounds__(128, 8) k_lists(const __grid_constant__ RebuildArgs R, long long ncells) {
+    await_previous();
     FN_GATED(R.gate);
     __shared__ int s_first[9 * 128];
     __shared__ unsigned char s_len[9 * 128];
@@ -1896,6 +1930,7 @@ __device__ __forceinline__ void block_scan_array(const int* v, int n, int* out, 
 }
 
 __global__ void __launch_bounds__(kBrickThreads) k_lists_brick(const RebuildArgs R, const int4* __restrict__ bricks) {
+    await_previous();
     FN_GATED(R.gate);
     __shared__ int s_cnt[kBrickHalo], s_start[kBrickHalo], s_coff[kBrickHalo + 1];
     __shared__ int s_icnt[kBrickCells], s_ioff[kBrickCells + 1];
@@ -2024,6 +2059,8 @@ __global__ void __launch_bounds__(kBrickThreads) k_lists_brick(const RebuildArgs
    csr + t * region (region >= beads per tile x list capacity), and their
    number in tile_items[t].  One block of at least the tile's bead count. */
 __global__ void k_list_tiles(const RebuildArgs R) {
+    await_previous();
+    let_next_start();
     FN_GATED(R.gate);
     __shared__ int ws[33];
     const FnTile t = R.tiles[blockIdx.x];
@@ -2077,6 +2114,8 @@ __device__ __forceinline__ int block_exclusive_scan(int v, int* warp_sums, int& 
 
 __global__ void __launch_bounds__(SCAN_THREADS) k_scan_partials(const int* in, long long n,
                                                                  int* block_sums, const int* gate) {
+    await_previous();
+    let_next_start();
     FN_GATED(gate);
     __shared__ int ws[33];
     const long long base = (long long)blockIdx.x * SCAN_TILE + (long long)threadIdx.x * SCAN_ITEMS;
@@ -2141,6 +2180,8 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan_apply_direct(const int* i
                                                                      const int* block_sums, int nblocks,
                                                                      int* out, int* grand_total,
                                                                      const int* gate, int* zero) {
+    await_previous();
+    let_next_start();
     FN_GATED(gate);
     __shared__ int ws[33];
     int before = 0;
@@ -2172,6 +2213,8 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan_apply_direct(const int* i
 /* Observables: deterministic two-pass FP64 reduction per network.           */
 
 __global__ void k_observe_partial(const ObserveArgs O) {
+    await_previous();
+    let_next_start();
     __shared__ double sx[256], sy[256], sz[256];
     __shared__ long long sb[256], sa[256];
     const int tid = threadIdx.x;
@@ -2244,11 +2287,30 @@ __device__ __forceinline__ void add_partials(const double* partial, int nblocks,
 }
 
 __global__ void k_observe_final(const double* partial, int nblocks, double* out) {
+    await_previous();
+    let_next_start();
     add_partials<5>(partial, nblocks, out);
 }
 
 /* ------------------------------------------------------------------------ */
 /* launch wrappers                                                           */
+
+/* Launches a kernel of the step sequence (await_previous) so that its blocks
+   may be placed while the kernel before it drains. */
+template <class... P, class... X>
+static void launch_next(void (*kernel)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t s, X... x) {
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, kernel, P(x)...); /* errors are read by the callers' cudaGetLastError */
+}
 
 static int step_flags(bool do_drift, bool store_v) {
     return FN_STEP_SPRINGS | FN_STEP_ANGLES | FN_STEP_CONTACTS | (do_drift ? FN_STEP_DRIFT : 0) |
@@ -2259,9 +2321,9 @@ cudaError_t launch_step(const StepArgs& A, int ntiles, int block, bool damp, boo
                         bool store_v, cudaStream_t s) {
     if (ntiles <= 0) return cudaSuccess;
     if (damp)
-        k_step<true><<<ntiles, block, 0, s>>>(A, step_flags(do_drift, store_v));
+        launch_next(k_step<true>, ntiles, block, 0, s, A, step_flags(do_drift, store_v));
     else
-        k_step<false><<<ntiles, block, 0, s>>>(A, step_flags(do_drift, store_v));
+        launch_next(k_step<false>, ntiles, block, 0, s, A, step_flags(do_drift, store_v));
     return cudaGetLastError();
 }
 
@@ -2297,13 +2359,13 @@ cudaError_t launch_step_tiled(const StepArgs& A, int ntiles, int block, bool dam
     const size_t sm = step_tiled_smem(A.max_tile_sp, A.max_tile_an);
     const int flags = step_flags(do_drift, store_v);
     if (damp && A.uniform)
-        k_step_tiled<true, true><<<ntiles, block, sm, s>>>(A, flags);
+        launch_next(k_step_tiled<true, true>, ntiles, block, sm, s, A, flags);
     else if (damp)
-        k_step_tiled<true, false><<<ntiles, block, sm, s>>>(A, flags);
+        launch_next(k_step_tiled<true, false>, ntiles, block, sm, s, A, flags);
     else if (A.uniform)
-        k_step_tiled<false, true><<<ntiles, block, sm, s>>>(A, flags);
+        launch_next(k_step_tiled<false, true>, ntiles, block, sm, s, A, flags);
     else
-        k_step_tiled<false, false><<<ntiles, block, sm, s>>>(A, flags);
+        launch_next(k_step_tiled<false, false>, ntiles, block, sm, s, A, flags);
     return cudaGetLastError();
 }
 
@@ -2329,13 +2391,13 @@ cudaError_t launch_step_chain(const StepArgs& A, int ntiles, int block, bool dam
     const size_t sm = step_chain_smem(block);
     const int flags = step_flags(do_drift, store_v);
     if (damp && A.uniform)
-        k_step_chain<true, false, true><<<ntiles, block, sm, s>>>(A, flags);
+        launch_next(k_step_chain<true, false, true>, ntiles, block, sm, s, A, flags);
     else if (damp)
-        k_step_chain<true, false, false><<<ntiles, block, sm, s>>>(A, flags);
+        launch_next(k_step_chain<true, false, false>, ntiles, block, sm, s, A, flags);
     else if (A.uniform)
-        k_step_chain<false, false, true><<<ntiles, block, sm, s>>>(A, flags);
+        launch_next(k_step_chain<false, false, true>, ntiles, block, sm, s, A, flags);
     else
-        k_step_chain<false, false, false><<<ntiles, block, sm, s>>>(A, flags);
+        launch_next(k_step_chain<false, false, false>, ntiles, block, sm, s, A, flags);
     return cudaGetLastError();
 }
 
@@ -2362,17 +2424,17 @@ cudaError_t launch_step_staged(const StepArgs& A, int ntiles, int block, bool da
     const size_t sm = step_staged_smem(block, A.chunk);
     if (damp) {
         if (do_drift)
-            k_step_staged<true, true, true><<<ntiles, block, sm, s>>>(A);
+            launch_next(k_step_staged<true, true, true>, ntiles, block, sm, s, A);
         else
-            k_step_staged<true, false, false><<<ntiles, block, sm, s>>>(A);
+            launch_next(k_step_staged<true, false, false>, ntiles, block, sm, s, A);
     } else {
         if (do_drift) {
             if (store_v)
-                k_step_staged<false, true, true><<<ntiles, block, sm, s>>>(A);
+                launch_next(k_step_staged<false, true, true>, ntiles, block, sm, s, A);
             else
-                k_step_staged<false, true, false><<<ntiles, block, sm, s>>>(A);
+                launch_next(k_step_staged<false, true, false>, ntiles, block, sm, s, A);
         } else {
-            k_step_staged<false, false, false><<<ntiles, block, sm, s>>>(A);
+            launch_next(k_step_staged<false, false, false>, ntiles, block, sm, s, A);
         }
     }
     return cudaGetLastError();
@@ -2381,16 +2443,16 @@ cudaError_t launch_step_staged(const StepArgs& A, int ntiles, int block, bool da
 
 cudaError_t launch_forces_chain(const StepArgs& A, int ntiles, int block, int terms, cudaStream_t s) {
     if (ntiles <= 0) return cudaSuccess;
-    k_step_chain<false, true, false><<<ntiles, block, step_chain_smem(block), s>>>(A, terms);
+    launch_next(k_step_chain<false, true, false>, ntiles, block, step_chain_smem(block), s, A, terms);
     return cudaGetLastError();
 }
 
 cudaError_t launch_drift(const StepArgs& A, int ntiles, int block, bool store_v, cudaStream_t s) {
     if (ntiles <= 0) return cudaSuccess;
     if (store_v)
-        k_drift<true><<<ntiles, block, 0, s>>>(A);
+        launch_next(k_drift<true>, ntiles, block, 0, s, A);
     else
-        k_drift<false><<<ntiles, block, 0, s>>>(A);
+        launch_next(k_drift<false>, ntiles, block, 0, s, A);
     return cudaGetLastError();
 }
 
@@ -2412,7 +2474,7 @@ long long scan_block_count(long long n) { return (n + SCAN_TILE - 1) / SCAN_TILE
 cudaError_t launch_exclusive_scan(const int* in, long long n, int* out, int* block_sums, cudaStream_t s) {
     if (n <= 0) return cudaSuccess;
     const long long nblk = scan_block_count(n);
-    k_scan_partials<<<(unsigned)nblk, SCAN_THREADS, 0, s>>>(in, n, block_sums, nullptr);
+    launch_next(k_scan_partials, nblk, SCAN_THREADS, 0, s, in, n, block_sums, nullptr);
     k_scan_sums<<<1, SCAN_THREADS, 0, s>>>(block_sums, (int)nblk, out + n, nullptr);
     k_scan_apply<<<(unsigned)nblk, SCAN_THREADS, 0, s>>>(in, n, block_sums, out, nullptr, nullptr);
     return cudaGetLastError();
@@ -2430,44 +2492,40 @@ template <int G>
 static void launch_lists_group(const RebuildArgs& R, int nb, long long ncells, cudaStream_t s) {
     constexpr int PER = 128 / G;
     if (R.uniform)
-        k_lists_group<G, true><<<(nb + PER - 1) / PER, 128, 0, s>>>(R, ncells);
+        launch_next(k_lists_group<G, true>, (nb + PER - 1) / PER, 128, 0, s, R, ncells);
     else
-        k_lists_group<G, false><<<(nb + PER - 1) / PER, 128, 0, s>>>(R, ncells);
+        launch_next(k_lists_group<G, false>, (nb + PER - 1) / PER, 128, 0, s, R, ncells);
 }
 
 cudaError_t launch_rebuild(const RebuildArgs& R, int ntiles, int block, int nb, long long ncells,
                            int* scan_block_sums, cudaStream_t s) {
-    cudaError_t e;
     const unsigned fill_blocks = (unsigned)std::min<long long>(4096, (ncells + 255) / 256 + 1);
     /* cell fills are cleared by the scan's last pass and list counts by
        k_cells, so only the cell counts need a pass of their own */
-    if (R.gate)
-        k_fill_int<<<fill_blocks, 256, 0, s>>>(R.cell_count, ncells, 0, R.gate);
-    else if ((e = cudaMemsetAsync(R.cell_count, 0, sizeof(int) * (size_t)ncells, s)))
-        return e;
-    if (ntiles > 0) k_cells<<<ntiles, block, 0, s>>>(R);
+    launch_next(k_fill_int, fill_blocks, 256, 0, s, R.cell_count, ncells, 0, R.gate);
+    if (ntiles > 0) launch_next(k_cells, ntiles, block, 0, s, R);
     const long long nblk = scan_block_count(ncells);
-    k_scan_partials<<<(unsigned)nblk, SCAN_THREADS, 0, s>>>(R.cell_count, ncells, scan_block_sums, R.gate);
-    k_scan_apply_direct<<<(unsigned)nblk, SCAN_THREADS, 0, s>>>(R.cell_count, ncells, scan_block_sums, (int)nblk,
+    launch_next(k_scan_partials, nblk, SCAN_THREADS, 0, s, R.cell_count, ncells, scan_block_sums, R.gate);
+    launch_next(k_scan_apply_direct, nblk, SCAN_THREADS, 0, s, R.cell_count, ncells, scan_block_sums, (int)nblk,
                                                                  R.cell_start, R.cell_start + ncells, R.gate,
                                                                  R.cell_fill);
-    if (nb > 0) k_scatter<<<(nb + 255) / 256, 256, 0, s>>>(R, nb);
-    k_cell_sort<<<(unsigned)((ncells + 255) / 256), 256, 0, s>>>(R, (int)ncells);
+    if (nb > 0) launch_next(k_scatter, (nb + 255) / 256, 256, 0, s, R, nb);
+    launch_next(k_cell_sort, (unsigned)((ncells + 255) / 256), 256, 0, s, R, (int)ncells);
     if (R.bricks) {
-        if (R.nbricks > 0) k_lists_brick<<<R.nbricks, kBrickThreads, 0, s>>>(R, R.bricks);
+        if (R.nbricks > 0) launch_next(k_lists_brick, R.nbricks, kBrickThreads, 0, s, R, R.bricks);
     } else if (nb > 0 && R.list_lanes == 8) {
         launch_lists_group<8>(R, nb, ncells, s);
     } else if (nb > 0 && nb <= kGroupedBeads) {
         launch_lists_group<4>(R, nb, ncells, s);
     } else if (nb > 0) {
         if (R.uniform)
-            k_lists<true><<<(nb + 127) / 128, 128, 0, s>>>(R, ncells);
+            launch_next(k_lists<true>, (nb + 127) / 128, 128, 0, s, R, ncells);
         else
-            k_lists<false><<<(nb + 127) / 128, 128, 0, s>>>(R, ncells);
+            launch_next(k_lists<false>, (nb + 127) / 128, 128, 0, s, R, ncells);
     }
     /* the staged step kernel's copy, one block per tile (tiles are at most
        block - 4 beads wide) */
-    if (R.csr && ntiles > 0) k_list_tiles<<<ntiles, block, 0, s>>>(R);
+    if (R.csr && ntiles > 0) launch_next(k_list_tiles, ntiles, block, 0, s, R);
     return cudaGetLastError();
 }
 
@@ -2475,6 +2533,8 @@ cudaError_t launch_rebuild(const RebuildArgs& R, int ntiles, int block, int nb, 
    threshold since the last rebuild (image positions, so wraps do not count). */
 __global__ void k_disp_check(const FnTile* tiles, const double4* img, const double4* ref, double thresh2,
                              int* gate) {
+    await_previous();
+    let_next_start();
     const FnTile t = tiles[blockIdx.x];
     const int i = t.begin + (int)threadIdx.x;
     if (i >= t.end) return;
@@ -2483,16 +2543,9 @@ __global__ void k_disp_check(const FnTile* tiles, const double4* img, const doub
     if (!(dx * dx + dy * dy + dz * dz <= thresh2)) *gate = 1;
 }
 
-/* After a gated rebuild: the new reference positions. */
-__global__ void k_ref_update(const FnTile* tiles, const double4* img, double4* ref, const int* gate) {
-    FN_GATED(gate);
-    const FnTile t = tiles[blockIdx.x];
-    const int i = t.begin + (int)threadIdx.x;
-    if (i >= t.end) return;
-    ref[i] = img[i];
-}
-
 __global__ void k_gate_clear(int* gate, unsigned long long* counters) {
+    await_previous();
+    let_next_start();
     if (*gate) {
         counters[FN_CNT_REBUILDS] += 1ull;
         *gate = 0;
@@ -2502,11 +2555,13 @@ __global__ void k_gate_clear(int* gate, unsigned long long* counters) {
 cudaError_t launch_verlet_rebuild(const RebuildArgs& R, const FnTile* tiles, const double4* img,
                                   double4* ref, double thresh2, int* gate, int ntiles, int block, int nb,
                                   long long ncells, int* scan_block_sums, cudaStream_t s) {
-    if (ntiles > 0) k_disp_check<<<ntiles, block, 0, s>>>(tiles, img, ref, thresh2, gate);
-    cudaError_t e = launch_rebuild(R, ntiles, block, nb, ncells, scan_block_sums, s);
+    if (ntiles > 0) launch_next(k_disp_check, ntiles, block, 0, s, tiles, img, ref, thresh2, gate);
+    RebuildArgs G = R;
+    G.img = img;
+    G.ref = ref;
+    cudaError_t e = launch_rebuild(G, ntiles, block, nb, ncells, scan_block_sums, s);
     if (e) return e;
-    if (ntiles > 0) k_ref_update<<<ntiles, block, 0, s>>>(tiles, img, ref, gate);
-    k_gate_clear<<<1, 1, 0, s>>>(gate, R.counters);
+    launch_next(k_gate_clear, 1, 1, 0, s, gate, R.counters);
     return cudaGetLastError();
 }
 
@@ -2605,6 +2660,7 @@ __device__ __forceinline__ void add_outer(double* w, double ax, double ay, doubl
    hide (measured on the 1M-bead tensile network: 0.37 ms per evaluation
    against 0.45 ms at the 102 registers the compiler picks unbounded). */
 __global__ void __launch_bounds__(256, 3) k_energy_partial(const EnergyArgs E) {
+    await_previous();
     __shared__ double red[8][FN_EN_N];
     const FnNet& N = E.nets[E.net];
     double acc[FN_EN_N];
@@ -2704,18 +2760,20 @@ __global__ void __launch_bounds__(256, 3) k_energy_partial(const EnergyArgs E) {
 }
 
 __global__ void k_energy_final(const double* partial, int nblocks, double* out) {
+    await_previous();
+    let_next_start();
     add_partials<FN_EN_N>(partial, nblocks, out);
 }
 
 cudaError_t launch_energy(const EnergyArgs& E, int nblocks, double* out, cudaStream_t s) {
-    k_energy_partial<<<nblocks, 256, 0, s>>>(E);
-    k_energy_final<<<1, 32 * FN_EN_N, 0, s>>>(E.partial, nblocks, out);
+    launch_next(k_energy_partial, nblocks, 256, 0, s, E);
+    launch_next(k_energy_final, 1, 32 * FN_EN_N, 0, s, E.partial, nblocks, out);
     return cudaGetLastError();
 }
 
 cudaError_t launch_observe(const ObserveArgs& O, int nblocks, double* out, cudaStream_t s) {
-    k_observe_partial<<<nblocks, 256, 0, s>>>(O);
-    k_observe_final<<<1, 32 * 5, 0, s>>>(O.partial, nblocks, out);
+    launch_next(k_observe_partial, nblocks, 256, 0, s, O);
+    launch_next(k_observe_final, 1, 32 * 5, 0, s, O.partial, nblocks, out);
     return cudaGetLastError();
 }
 

@@ -215,6 +215,8 @@ struct RebuildArgs {
     unsigned long long* counters;
     int n_nets;
     const int* gate; /* displacement mode: rebuild only when *gate != 0 */
+    const double4* img; /* and take these positions as the new reference */
+    double4* ref;
     /* bricks of the staged list build: network, first cell x, y, z (null:
        the per-bead list build) */
     const int4* bricks;

@@ -795,8 +795,9 @@ int build_bricks(fn_ctx* c) {
 
 /* Block size (and, for the staged chain kernel, contact items per thread and
    round) of the step kernel: tiles, per-tile tables and kernel attributes.
-   items_per_thread 0 selects the plain chain kernel. */
-int set_block(fn_ctx* c, int block, int items_per_thread) {
+   items_per_thread 0 selects the plain chain kernel; `wide` its form with
+   five warps per 28 beads, for contexts small enough. */
+int set_block(fn_ctx* c, int block, int items_per_thread, bool wide = false) {
     if (c->chain && block > fn::kChainMaxBlock)
         return fail(c, FN_ERR_ARG, "block size " + std::to_string(block) + ": the chain step kernel takes at most " +
                                        std::to_string(fn::kChainMaxBlock) + " threads per block");
@@ -844,6 +845,7 @@ int set_block(fn_ctx* c, int block, int items_per_thread) {
     CK(cudaStreamSynchronize(c->stream));
     c->ntiles = n;
     c->block = block;
+    c->wide = wide && c->chain && !c->staged && c->nb <= fn::kWideContext;
     return FN_OK;
 }
 
@@ -902,6 +904,7 @@ fn::StepArgs step_args(fn_ctx* c, bool pingpong) {
     A.ch_flags = c->ch_flags.p;
     A.ch_status = c->ch_status.p;
     A.nb = (int)c->nb;
+    A.wide = c->wide ? 1 : 0;
     A.uniform = c->uniform ? 1 : 0;
     if (c->uniform) {
         A.net0 = c->nets_h[0];
@@ -1561,7 +1564,7 @@ static int upload_host(fn_ctx* c, int n_networks, const fn_network_desc* nets) {
     int r = build_bricks(c);
     if (r) return r;
     r = set_block(c, c->cfg.block_size > 0 ? c->cfg.block_size : 128,
-                  c->cfg.chain_mode == 0 ? kDefaultItemsPerThread : 0);
+                  c->cfg.chain_mode == 0 ? kDefaultItemsPerThread : 0, c->cfg.block_size == 0);
     if (r) return r;
     r = verlet_setup(c);
     if (r) return r;
@@ -1842,7 +1845,8 @@ static int upload_device(fn_ctx* c, int n_networks, const fn_network_desc* nets)
     c->uploaded_on_device = true;
     r = build_bricks(c);
     if (r) return r;
-    r = set_block(c, c->cfg.block_size > 0 ? c->cfg.block_size : 128, c->cfg.chain_mode == 0 ? kDefaultItemsPerThread : 0);
+    r = set_block(c, c->cfg.block_size > 0 ? c->cfg.block_size : 128, c->cfg.chain_mode == 0 ? kDefaultItemsPerThread : 0,
+                  c->cfg.block_size == 0);
     if (r) return r;
     r = verlet_setup(c);
     if (r) return r;
@@ -2558,7 +2562,8 @@ FN_API int fn_autotune(fn_ctx* c, int steps_per_trial) {
     const long long steps0 = c->steps_done, rb0 = c->rebuilds_done;
     const bool timing0 = c->timing;
     c->timing = false;
-    std::vector<std::pair<int, int>> shapes;
+    std::vector<std::pair<int, int>> shapes; /* block, items per thread (-1: the wide form) */
+    if (c->chain && c->nb <= fn::kWideContext) shapes.emplace_back(128, -1);
     for (int b : {64, 96, 128, 192, 256, 384, 512}) {
         if (c->chain && b > fn::kChainMaxBlock) continue;
         if (c->chain && c->cfg.chain_mode == 0)
@@ -2568,14 +2573,14 @@ FN_API int fn_autotune(fn_ctx* c, int steps_per_trial) {
     int dev = 0, optin = 0;
     CK(cudaGetDevice(&dev));
     CK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-    std::pair<int, int> best{c->block, c->staged ? c->chunk / c->block : 0};
+    std::pair<int, int> best{c->block, c->wide ? -1 : c->staged ? c->chunk / c->block : 0};
     float best_ms = 1e30f;
     cudaEvent_t e0, e1;
     CK(cudaEventCreate(&e0));
     CK(cudaEventCreate(&e1));
     for (const auto& sh : shapes) {
         if (sh.second > 0 && fn::step_staged_smem(sh.first, sh.first * sh.second) > (size_t)optin) continue;
-        if ((r = set_block(c, sh.first, sh.second))) break;
+        if ((r = set_block(c, sh.first, std::max(sh.second, 0), sh.second < 0))) break;
         for (int rep = 0; rep < 2 && !r; ++rep) { /* first run warms up */
             c->cur = cur0;
             for (auto& sn : snaps)
@@ -2596,7 +2601,7 @@ FN_API int fn_autotune(fn_ctx* c, int steps_per_trial) {
     /* then the list build (bead by bead, by bricks, by groups of lanes) at
        that shape */
     int best_build = c->list_build;
-    if (!r && (r = set_block(c, best.first, best.second)) == 0) {
+    if (!r && (r = set_block(c, best.first, std::max(best.second, 0), best.second < 0)) == 0) {
         float ms_build[3] = {1e30f, 1e30f, 1e30f};
         for (int mode = 0; mode < 3 && !r; ++mode) {
             c->list_build = mode;
@@ -2631,7 +2636,7 @@ FN_API int fn_autotune(fn_ctx* c, int steps_per_trial) {
     c->rebuilds_done = rb0;
     c->timing = timing0;
     if (r) return r;
-    return set_block(c, best.first, best.second);
+    return set_block(c, best.first, std::max(best.second, 0), best.second < 0);
     FN_CATCH(c)
 }
 

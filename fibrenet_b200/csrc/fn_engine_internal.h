@@ -102,6 +102,7 @@ struct fn_ctx {
     /* staged chain step kernel: tile-compacted contact list, items per tile,
        contact items staged per round */
     bool staged = false;
+    bool wide = false; /* the chain kernel's form with five warps per 28 beads */
     int chunk = 0;
     long long csr_region = 0;
     DevBuf<int> csr, tile_items;

@@ -341,19 +341,21 @@ enum { FN_STEP_SPRINGS = 1, FN_STEP_ANGLES = 2, FN_STEP_CONTACTS = 4, FN_STEP_DR
 
 /* AdvanceVelocity and the next AdvancePosition for bead i with its complete
    force (Fx, Fy, Fz), then the stores. */
+/* What the kick reads of bead i: its image position, force and velocity_old. */
+struct KickState {
+    double4 im;
+    float4 fo, vo;
+};
+
+__device__ __forceinline__ KickState kick_state(const StepArgs& A, int i) {
+    return KickState{A.img_in[i], A.force[i], A.vold[i]};
+}
+
 template <bool DAMP>
 __device__ __forceinline__ void kick_drift(const StepArgs& A, const FnNet& N, int i, double4 p, double Fx, double Fy,
-                                           double Fz, bool do_drift, bool store_v) {
-    /* late: the next step's blocks take shared memory and slots from this one's
-       (60k beads: 19.1 us per step, 20.2 with this at the kernel's start) */
-    let_next_start();
-    /* loaded before the finiteness test: behind its branch these loads, and
-       with them every load of the kernel that reaches DRAM, take twice as
-       long (1M-bead tensile step 204 us against 108, the same sectors, hits
-       and DRAM bytes; networks that fit L2 see no difference) */
-    double4 im = A.img_in[i];
-    const float4 fo = A.force[i];
-    const float4 vo = A.vold[i];
+                                           double Fz, KickState k, bool do_drift, bool store_v) {
+    double4 im = k.im;
+    const float4 fo = k.fo, vo = k.vo;
     const float fx = (float)Fx, fy = (float)Fy, fz = (float)Fz;
     if (!(isfinite(fx) && isfinite(fy) && isfinite(fz)))
         atomicAdd(A.counters + FN_CNT_NONFINITE, 1ull);
@@ -402,7 +404,15 @@ __device__ __forceinline__ void finish_bead(const StepArgs& A, const FnNet& N, i
             Fz += Rz;
         }
     }
-    kick_drift<DAMP>(A, N, i, p, Fx, Fy, Fz, (flags & FN_STEP_DRIFT) != 0, DAMP || (flags & FN_STEP_STORE_V));
+    /* late: the next step's blocks take shared memory and slots from this one's
+       (60k beads: 19.1 us per step, 20.2 with this at the kernel's start) */
+    let_next_start();
+    /* loaded before the finiteness test: behind its branch these loads, and
+       with them every load of the kernel that reaches DRAM, take twice as
+       long (1M-bead tensile step 204 us against 108, the same sectors, hits
+       and DRAM bytes; networks that fit L2 see no difference) */
+    const KickState state = kick_state(A, i);
+    kick_drift<DAMP>(A, N, i, p, Fx, Fy, Fz, state, (flags & FN_STEP_DRIFT) != 0, DAMP || (flags & FN_STEP_STORE_V));
 }
 
 template <bool DAMP>
@@ -604,6 +614,48 @@ __device__ __forceinline__ int block_scan_any(int v, int* warp_sums, int& total)
     return r;
 }
 
+/* The spring from a bead to the next one, (x, y, z) apart (kernel.cl:377-424):
+   their distance l and its inverse, the force on the bead, and the bead's
+   status after the step. */
+__device__ __forceinline__ void chain_spring(unsigned fl, unsigned st0, float4 par, bool wanted, double x, double y,
+                                             double z, double& l, double& il, double& gx, double& gy, double& gz,
+                                             unsigned& st) {
+    root_and_inverse(x * x + y * y + z * z, l, il);
+    if ((fl & FN_CH_SPRING) && (st0 & 1) && !(fl & FN_CH_SP_INERT)) {
+        double factor = (double)par.x - l;
+        if ((fl & FN_CH_SP_FL) && fabs(-(double)par.z * factor * il) > (double)par.w) {
+            st &= ~1u; /* breaks: no force from this step on (kernel.cl:391-397) */
+        } else if (wanted) {
+            factor *= (double)par.y;
+            gx = x * il * factor;
+            gy = y * il * factor;
+            gz = z * il * factor;
+        }
+    }
+}
+
+/* A bead's bonded terms in ascending bond order: previous spring, next spring
+   (f: its slot of the springs' forces), angles centred on the previous bead,
+   on itself (cx, cy, cz) and on the next one (o: its slot of the angles'). */
+__device__ __forceinline__ void chain_gather(const double* f, const double* o, double cx, double cy, double cz,
+                                             double& Fx, double& Fy, double& Fz) {
+    Fx -= f[-3];
+    Fy -= f[-2];
+    Fz -= f[-1];
+    Fx += f[0];
+    Fy += f[1];
+    Fz += f[2];
+    Fx += o[-3];
+    Fy += o[-2];
+    Fz += o[-1];
+    Fx += cx;
+    Fy += cy;
+    Fz += cz;
+    Fx += o[6];
+    Fy += o[7];
+    Fz += o[8];
+}
+
 /* Step kernel for networks in chain form (every spring joins consecutive
    beads j, j+1 and every angle is centred on its middle bead, as fibres
    are).  Thread t of a block works for bead j = tile begin - 2 + t (the tile
@@ -671,19 +723,8 @@ __global__ void __launch_bounds__(kChainMaxBlock, 4) k_step_chain(const __grid_c
         x -= s_img[3 * tid + 3];
         y -= s_img[3 * tid + 4];
         z -= s_img[3 * tid + 5];
-        root_and_inverse(x * x + y * y + z * z, l, il);
-        if ((fl & FN_CH_SPRING) && (st0 & 1) && !(fl & FN_CH_SP_INERT)) {
-            const float4 sp = A.ch_sp[i];
-            double factor = (double)sp.x - l;
-            if ((fl & FN_CH_SP_FL) && fabs(-(double)sp.z * factor * il) > (double)sp.w) {
-                st &= ~1u; /* breaks: no force from this step on (kernel.cl:391-397) */
-            } else if (!FORCES_ONLY || (flags & FN_STEP_SPRINGS)) {
-                factor *= (double)sp.y;
-                gx = x * il * factor;
-                gy = y * il * factor;
-                gz = z * il * factor;
-            }
-        }
+        chain_spring(fl, st0, (fl & FN_CH_SPRING) ? A.ch_sp[i] : make_float4(0.f, 0.f, 0.f, 0.f),
+                     !FORCES_ONLY || (flags & FN_STEP_SPRINGS), x, y, z, l, il, gx, gy, gz, st);
         s_len[tid] = make_double2(l, il);
         s_spf[3 * tid] = gx;
         s_spf[3 * tid + 1] = gy;
@@ -730,23 +771,7 @@ __global__ void __launch_bounds__(kChainMaxBlock, 4) k_step_chain(const __grid_c
     if (active) {
         p = A.pos_in[i];
         if (!FORCES_ONLY) base_force<DAMP>(A, N, i, p, Fx, Fy, Fz);
-        const double* f = s_spf + 3 * tid;
-        Fx -= f[-3];
-        Fy -= f[-2];
-        Fz -= f[-1];
-        Fx += f[0];
-        Fy += f[1];
-        Fz += f[2];
-        const double* o = s_ang + 6 * tid;
-        Fx += o[-3];
-        Fy += o[-2];
-        Fz += o[-1];
-        Fx += cx;
-        Fy += cy;
-        Fz += cz;
-        Fx += o[6];
-        Fy += o[7];
-        Fz += o[8];
+        chain_gather(s_spf + 3 * tid, s_ang + 6 * tid, cx, cy, cz, Fx, Fy, Fz);
         if (!FORCES_ONLY || (flags & FN_STEP_CONTACTS)) {
             nc = A.list_count[i];
             if (nc > A.list_cap) nc = A.list_cap;
@@ -866,7 +891,182 @@ __global__ void __launch_bounds__(kChainMaxBlock, 4) k_step_chain(const __grid_c
         A.force[i] = make_float4((float)Fx, (float)Fy, (float)Fz, 0.0f);
         return;
     }
-    kick_drift<DAMP>(A, N, i, p, Fx, Fy, Fz, (flags & FN_STEP_DRIFT) != 0, DAMP || (flags & FN_STEP_STORE_V));
+    let_next_start();
+    const KickState state = kick_state(A, i); /* before the finiteness test, as in finish_bead */
+    kick_drift<DAMP>(A, N, i, p, Fx, Fy, Fz, state, (flags & FN_STEP_DRIFT) != 0, DAMP || (flags & FN_STEP_STORE_V));
+}
+
+/* The chain step for small contexts, five warps per 28 beads at most: one warp
+   evaluates the bonds (thread t for bead begin - 2 + t, as in k_step_chain)
+   while four others evaluate the contacts, four lanes per bead and
+   kWideItems contacts at a time into shared memory; then the first warp adds
+   them to its beads' forces in list order and moves the beads.  The terms and
+   their order are k_step_chain's, so the bits are.
+   A bead's step is then a few dependent loads and one or two contacts deep
+   instead of as many as its warp's longest list, and the bonds' chain of roots
+   and the arc cosine runs beside it: small networks wait for those chains (10k
+   beads 9.6 -> 4.3 us per step). */
+constexpr int kWideBeads = 28, kWideItems = 16, kWideThreads = 160;
+
+/* A barrier of the block's five warps, reached from the code of either role;
+   true when `p` is on any thread. */
+__device__ __forceinline__ bool wide_barrier_or(bool p) {
+    int any;
+    asm volatile(
+        "{\n .reg .pred a, b;\n setp.ne.s32 a, %1, 0;\n barrier.cta.red.or.pred b, 1, %2, a;\n selp.s32 %0, 1, 0, b;\n}"
+        : "=r"(any)
+        : "r"((int)p), "n"(kWideThreads)
+        : "memory");
+    return any != 0;
+}
+__device__ __forceinline__ void wide_barrier() {
+    asm volatile("barrier.cta.sync 2, %0;" ::"n"(kWideThreads) : "memory");
+}
+
+template <bool DAMP, bool UNIFORM>
+__global__ void __launch_bounds__(kWideThreads, 6) k_step_wide(const __grid_constant__ StepArgs A, int flags, int parts,
+                                                               int width) {
+    __shared__ double s_img[3 * 32], s_spf[3 * 33], s_ang[6 * 33];
+    __shared__ double2 s_len[32];
+    __shared__ double s_R[kWideBeads * (3 * kWideItems + 1)];
+    __shared__ unsigned char s_Rf[kWideBeads * kWideItems], s_ok[32];
+    const FnTile tile = A.tiles[blockIdx.x / parts];
+    const int begin = tile.begin + (blockIdx.x % parts) * width;
+    const int n = min(tile.end - begin, width); /* may be <= 0: nothing to do */
+    const int tid = threadIdx.x;
+    const FnNet& N = UNIFORM ? A.net0 : A.nets[tile.net];
+    await_previous();
+    if (tid >= 32) {
+        const int b = (tid - 32) >> 2, g = tid & 3;
+        const int i = begin + b;
+        int nc = 0;
+        double4 p = make_double4(0.0, 0.0, 0.0, 0.0);
+        if (b < n) {
+            nc = min(A.list_count[i], A.list_cap);
+            p = A.pos_in[i];
+        }
+        double* R = s_R + b * (3 * kWideItems + 1);
+        unsigned char* Rf = s_Rf + b * kWideItems;
+        for (int k0 = 0;; k0 += kWideItems) {
+            const int k1 = min(nc, k0 + kWideItems);
+            /* two items at a time, their loads together */
+            for (int k = k0 + g; k < k1; k += 8) {
+                const int* row = A.list + (size_t)k * A.list_stride + i;
+                const bool two = k + 4 < k1;
+                const int j0 = row[0];
+                const int j1 = two ? row[4 * (size_t)A.list_stride] : j0;
+                const double4 q0 = A.pos_in[j0], q1 = A.pos_in[j1];
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    if (h == 1 && !two) break;
+                    const double4 q = h == 0 ? q0 : q1;
+                    double Rx = 0.0, Ry = 0.0, Rz = 0.0;
+                    const int acts = UNIFORM ? contact_force(N, A.pair0, p, q, Rx, Ry, Rz)
+                                             : contact_eval(N, A.pairs, p, q, Rx, Ry, Rz);
+                    const int at = k - k0 + 4 * h;
+                    R[3 * at] = Rx;
+                    R[3 * at + 1] = Ry;
+                    R[3 * at + 2] = Rz;
+                    Rf[at] = (unsigned char)acts;
+                }
+            }
+            if (!wide_barrier_or(nc > k0 + kWideItems)) break;
+            wide_barrier(); /* added: the next items may overwrite them */
+        }
+        return;
+    }
+
+    const int i = begin - 2 + tid; /* this thread's bead */
+    const bool active = tid >= 2 && tid < n + 2;
+    unsigned fl = 0, st0 = 0;
+    double x = 0.0, y = 0.0, z = 0.0;
+    float4 sp = make_float4(0.f, 0.f, 0.f, 0.f);
+    float2 an = make_float2(0.f, 0.f);
+    KickState state{};
+    double4 p = make_double4(0.0, 0.0, 0.0, 0.0);
+    int nc = 0;
+    if (tid < n + 4 && i >= 0 && i < A.nb) {
+        state.im = A.img_in[i];
+        x = state.im.x;
+        y = state.im.y;
+        z = state.im.z;
+        fl = A.ch_flags[i];
+        st0 = A.ch_status[i];
+        sp = A.ch_sp[i];
+        an = A.ch_an[i];
+        if (active) {
+            nc = min(A.list_count[i], A.list_cap);
+            p = A.pos_in[i];
+        }
+    }
+    s_img[3 * tid] = x;
+    s_img[3 * tid + 1] = y;
+    s_img[3 * tid + 2] = z;
+    __syncwarp();
+    double l = 0.0, il = 0.0, gx = 0.0, gy = 0.0, gz = 0.0;
+    unsigned st = st0;
+    if (tid < n + 3) {
+        x -= s_img[3 * tid + 3];
+        y -= s_img[3 * tid + 4];
+        z -= s_img[3 * tid + 5];
+        chain_spring(fl, st0, sp, true, x, y, z, l, il, gx, gy, gz, st);
+        s_len[tid] = make_double2(l, il);
+    }
+    s_spf[3 * tid] = gx;
+    s_spf[3 * tid + 1] = gy;
+    s_spf[3 * tid + 2] = gz;
+    s_ok[tid] = (unsigned char)((fl & FN_CH_SPRING) && (st & 1));
+    __syncwarp();
+    double cx = 0.0, cy = 0.0, cz = 0.0;
+    {
+        double pax = 0.0, pay = 0.0, paz = 0.0, pcx = 0.0, pcy = 0.0, pcz = 0.0;
+        if (tid >= 1 && tid < n + 3 && (fl & FN_CH_ANGLE) && (st0 & 2)) {
+            if ((fl & FN_CH_AN_FL) && !(s_ok[tid - 1] && s_ok[tid])) {
+                st &= ~2u; /* kernel.cl:278-284 */
+            } else {
+                const double* q = s_img + 3 * tid;
+                const double2 lp = s_len[tid - 1];
+                angle_arms(q[-3] - q[0], q[-2] - q[1], q[-1] - q[2], x, y, z, lp.x, lp.y, l, il, an, pax, pay, paz,
+                           pcx, pcy, pcz);
+                cx = -pax - pcx;
+                cy = -pay - pcy;
+                cz = -paz - pcz;
+            }
+        }
+        double* o = s_ang + 6 * tid;
+        o[0] = pax;
+        o[1] = pay;
+        o[2] = paz;
+        o[3] = pcx;
+        o[4] = pcy;
+        o[5] = pcz;
+    }
+    __syncwarp();
+    double Fx = 0.0, Fy = 0.0, Fz = 0.0;
+    if (active) {
+        state.fo = A.force[i];
+        state.vo = A.vold[i];
+        base_force<DAMP>(A, N, i, p, Fx, Fy, Fz);
+        chain_gather(s_spf + 3 * tid, s_ang + 6 * tid, cx, cy, cz, Fx, Fy, Fz);
+    }
+    const double* R = s_R + (tid - 2) * (3 * kWideItems + 1);
+    const unsigned char* Rf = s_Rf + (tid - 2) * kWideItems;
+    for (int k0 = 0;; k0 += kWideItems) {
+        const bool more = wide_barrier_or(false);
+        const int m = min(nc - k0, kWideItems);
+        for (int k = 0; k < m; ++k)
+            if (Rf[k]) {
+                Fx += R[3 * k];
+                Fy += R[3 * k + 1];
+                Fz += R[3 * k + 2];
+            }
+        if (!more) break;
+        wide_barrier();
+    }
+    let_next_start();
+    if (!active) return;
+    if (st != st0) A.ch_status[i] = (unsigned char)st;
+    kick_drift<DAMP>(A, N, i, p, Fx, Fy, Fz, state, (flags & FN_STEP_DRIFT) != 0, DAMP || (flags & FN_STEP_STORE_V));
 }
 
 /* ------------------------------------------------------------------------ */
@@ -2390,6 +2590,18 @@ cudaError_t launch_step_chain(const StepArgs& A, int ntiles, int block, bool dam
     if (ntiles <= 0) return cudaSuccess;
     const size_t sm = step_chain_smem(block);
     const int flags = step_flags(do_drift, store_v);
+    if (A.wide) {
+        const int parts = (block - 4 + kWideBeads - 1) / kWideBeads, width = (block - 4 + parts - 1) / parts;
+        if (damp && A.uniform)
+            launch_next(k_step_wide<true, true>, ntiles * parts, kWideThreads, 0, s, A, flags, parts, width);
+        else if (damp)
+            launch_next(k_step_wide<true, false>, ntiles * parts, kWideThreads, 0, s, A, flags, parts, width);
+        else if (A.uniform)
+            launch_next(k_step_wide<false, true>, ntiles * parts, kWideThreads, 0, s, A, flags, parts, width);
+        else
+            launch_next(k_step_wide<false, false>, ntiles * parts, kWideThreads, 0, s, A, flags, parts, width);
+        return cudaGetLastError();
+    }
     if (damp && A.uniform)
         launch_next(k_step_chain<true, false, true>, ntiles, block, sm, s, A, flags);
     else if (damp)

@@ -115,7 +115,9 @@ typedef struct fn_config {
     int reorder;        /* 1: renumber beads in Morton order of their fibre */
     int use_graphs;     /* 1: replay steps as CUDA graphs */
     int block_size;     /* threads per block for the step kernel; 0 = default
-                           (128); at most 256 on the chain path */
+                           (128, and on the chain path contexts of at most
+                           50,000 beads step with five warps per 28 beads);
+                           at most 256 on the chain path */
     int chain_mode;     /* 0 auto: per-bead bond records when the model is in
                            chain form (fibres), the tile's data staged in
                            shared memory before use; 1 chain form without

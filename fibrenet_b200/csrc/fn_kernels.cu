@@ -1576,20 +1576,8 @@ __device__ __forceinline__ void cell_sort_small(const float4* raw, int n, int* b
         }
 }
 
-/* Orders each cell's beads by index (the order a one-thread FillGrid sweep
-   would store them in) and drops the ones beyond the cell capacity, like the
-   `old < GRID_TAIL_SIZE` test of kernel.cl:503.  One thread per cell: cells
-   hold about one bead, and a warp's cells are one run of both arrays (counting
-   each bead's rank with the bead's own thread reads its cell at random: 188 us
-   against 52 on the 4M-bead mat). */
-__global__ void k_cell_sort(const __grid_constant__ RebuildArgs R, int ncells) {
-    await_previous();
-    let_next_start();
-    FN_GATED(R.gate);
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= ncells) return;
-    const int n = R.cell_count[c];
-    if (n == 0) return;
+/* One cell of n > 0 beads. */
+__device__ __forceinline__ void cell_sort_one(const RebuildArgs& R, int c, int n) {
     const int start = R.cell_start[c];
     const float4* raw = R.cell_raw + start;
     int* b = R.cell_beads + start;
@@ -1625,6 +1613,35 @@ __global__ void k_cell_sort(const __grid_constant__ RebuildArgs R, int ncells) {
         for (int k = R.cell_cap; k < n; ++k) R.cell_of[b[k]] = -1;
         atomicAdd(R.counters + FN_CNT_CELL_OVERFLOW, (unsigned long long)(n - R.cell_cap));
     }
+}
+
+/* Orders each cell's beads by index (the order a one-thread FillGrid sweep
+   would store them in) and drops the ones beyond the cell capacity, like the
+   `old < GRID_TAIL_SIZE` test of kernel.cl:503.  One thread per cell: cells
+   hold about one bead, and a warp's cells are one run of both arrays (counting
+   each bead's rank with the bead's own thread reads its cell at random: 188 us
+   against 52 on the 4M-bead mat). */
+__global__ void k_cell_sort(const __grid_constant__ RebuildArgs R, int ncells) {
+    await_previous();
+    let_next_start();
+    FN_GATED(R.gate);
+    const int c = blockIdx.x * blockDim.x + threadIdx.x;
+    if (c >= ncells) return;
+    const int n = R.cell_count[c];
+    if (n > 0) cell_sort_one(R, c, n);
+}
+
+/* The same for grids of mostly empty cells: one thread per bead in the grid, of
+   which the one at its cell's first place sorts the cell. */
+__global__ void k_cell_sort_sparse(const __grid_constant__ RebuildArgs R, int nb, long long ncells) {
+    await_previous();
+    let_next_start();
+    FN_GATED(R.gate);
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= nb || t >= R.cell_start[ncells]) return;
+    const int c = R.cell_of[__float_as_int(R.cell_raw[t].w)];
+    /* -1: dropped by its overfull cell's first thread just now */
+    if (c >= 0 && R.cell_start[c] == t) cell_sort_one(R, c, R.cell_count[c]);
 }
 
 /* BuildContactList's test (kernel.cl:574-586, 630-659) once the (minimum-
@@ -2278,11 +2295,64 @@ __global__ void k_list_tiles(const RebuildArgs R) {
 }
 
 /* ------------------------------------------------------------------------ */
-/* Exclusive scan of int counts (1024 threads x 2 items per block).          */
+/* Exclusive scan of int counts (1024 threads x ITEMS items per block).
+   The direct last pass adds up the sums of all blocks before its own: with 2
+   items per thread that work and the 4-byte loads took 260 us on the 32M
+   cells of 64 batched networks, with 8 and 16-byte loads 130 (the 4M-bead
+   mat's whole rebuild 930 -> 904 us); below 2M cells the smaller tile keeps
+   more SMs busy (10k beads, 100k cells: 27 us against 29).                   */
 
 constexpr int SCAN_THREADS = 1024;
-constexpr int SCAN_ITEMS = 2;
-constexpr int SCAN_TILE = SCAN_THREADS * SCAN_ITEMS;
+constexpr long long SCAN_SMALL = 2 << 20; /* cells from which on a thread takes 8 */
+
+static inline int scan_items(long long n) { return n >= SCAN_SMALL ? 8 : 2; }
+
+template <int SCAN_ITEMS>
+__device__ __forceinline__ void scan_load(const int* in, long long base, long long n, int* v) {
+    if (SCAN_ITEMS % 4 == 0 && base + SCAN_ITEMS <= n && ((uintptr_t)in & 15) == 0) {
+#pragma unroll
+        for (int k = 0; k < SCAN_ITEMS; k += 4) {
+            const int4 q = *reinterpret_cast<const int4*>(in + base + k);
+            v[k] = q.x;
+            v[k + 1] = q.y;
+            v[k + 2] = q.z;
+            v[k + 3] = q.w;
+        }
+    } else {
+#pragma unroll
+        for (int k = 0; k < SCAN_ITEMS; ++k) v[k] = base + k < n ? in[base + k] : 0;
+    }
+}
+
+template <int SCAN_ITEMS>
+__device__ __forceinline__ void scan_store(int* out, long long base, long long n, const int* v) {
+    if (SCAN_ITEMS % 4 == 0 && base + SCAN_ITEMS <= n && ((uintptr_t)out & 15) == 0) {
+#pragma unroll
+        for (int k = 0; k < SCAN_ITEMS; k += 4)
+            *reinterpret_cast<int4*>(out + base + k) = make_int4(v[k], v[k + 1], v[k + 2], v[k + 3]);
+    } else {
+#pragma unroll
+        for (int k = 0; k < SCAN_ITEMS; ++k)
+            if (base + k < n) out[base + k] = v[k];
+    }
+}
+
+/* Writes the exclusive sums of v, starting from ex; clears zero alongside. */
+template <int SCAN_ITEMS>
+__device__ __forceinline__ void scan_finish(int* out, int* zero, long long base, long long n, int* v, int ex) {
+#pragma unroll
+    for (int k = 0; k < SCAN_ITEMS; ++k) {
+        const int c = v[k];
+        v[k] = ex;
+        ex += c;
+    }
+    scan_store<SCAN_ITEMS>(out, base, n, v);
+    if (zero) {
+#pragma unroll
+        for (int k = 0; k < SCAN_ITEMS; ++k) v[k] = 0;
+        scan_store<SCAN_ITEMS>(zero, base, n, v);
+    }
+}
 
 __device__ __forceinline__ int block_exclusive_scan(int v, int* warp_sums, int& total) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -2312,17 +2382,18 @@ __device__ __forceinline__ int block_exclusive_scan(int v, int* warp_sums, int& 
     return r;
 }
 
+template <int SCAN_ITEMS>
 __global__ void __launch_bounds__(SCAN_THREADS) k_scan_partials(const int* in, long long n,
                                                                  int* block_sums, const int* gate) {
     await_previous();
     let_next_start();
     FN_GATED(gate);
     __shared__ int ws[33];
-    const long long base = (long long)blockIdx.x * SCAN_TILE + (long long)threadIdx.x * SCAN_ITEMS;
-    int s = 0;
+    const long long base = (long long)blockIdx.x * (SCAN_THREADS * SCAN_ITEMS) + (long long)threadIdx.x * SCAN_ITEMS;
+    int v[SCAN_ITEMS], s = 0;
+    scan_load<SCAN_ITEMS>(in, base, n, v);
 #pragma unroll
-    for (int k = 0; k < SCAN_ITEMS; ++k)
-        if (base + k < n) s += in[base + k];
+    for (int k = 0; k < SCAN_ITEMS; ++k) s += v[k];
     int total;
     block_exclusive_scan(s, ws, total);
     if (threadIdx.x == 0) block_sums[blockIdx.x] = total;
@@ -2347,35 +2418,28 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan_sums(int* block_sums, int
 
 /* Exclusive scan, last pass: each block's offset added, written to out;
    zero (if given) is cleared alongside, sparing a launch. */
+template <int SCAN_ITEMS>
 __global__ void __launch_bounds__(SCAN_THREADS) k_scan_apply(const int* in, long long n,
                                                               const int* block_sums, int* out,
                                                               const int* gate, int* zero) {
     FN_GATED(gate);
     __shared__ int ws[33];
-    const long long base = (long long)blockIdx.x * SCAN_TILE + (long long)threadIdx.x * SCAN_ITEMS;
+    const long long base = (long long)blockIdx.x * (SCAN_THREADS * SCAN_ITEMS) + (long long)threadIdx.x * SCAN_ITEMS;
     int v[SCAN_ITEMS];
     int s = 0;
+    scan_load<SCAN_ITEMS>(in, base, n, v);
 #pragma unroll
-    for (int k = 0; k < SCAN_ITEMS; ++k) {
-        v[k] = base + k < n ? in[base + k] : 0;
-        s += v[k];
-    }
+    for (int k = 0; k < SCAN_ITEMS; ++k) s += v[k];
     int total;
-    int ex = block_exclusive_scan(s, ws, total) + block_sums[blockIdx.x];
-#pragma unroll
-    for (int k = 0; k < SCAN_ITEMS; ++k) {
-        if (base + k < n) {
-            out[base + k] = ex;
-            if (zero) zero[base + k] = 0;
-        }
-        ex += v[k];
-    }
+    const int ex = block_exclusive_scan(s, ws, total) + block_sums[blockIdx.x];
+    scan_finish<SCAN_ITEMS>(out, zero, base, n, v, ex);
 }
 
 /* Exclusive scan, last pass, without a pass of its own over the block sums:
    each block adds up the raw sums of the blocks before it (a few thousand at
    most, read from L2), the last block writes the grand total; zero (if
    given) is cleared alongside. */
+template <int SCAN_ITEMS>
 __global__ void __launch_bounds__(SCAN_THREADS) k_scan_apply_direct(const int* in, long long n,
                                                                      const int* block_sums, int nblocks,
                                                                      int* out, int* grand_total,
@@ -2388,24 +2452,15 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan_apply_direct(const int* i
     for (int b = threadIdx.x; b < (int)blockIdx.x; b += SCAN_THREADS) before += block_sums[b];
     int offset;
     block_exclusive_scan(before, ws, offset); /* offset: the block sums' total */
-    const long long base = (long long)blockIdx.x * SCAN_TILE + (long long)threadIdx.x * SCAN_ITEMS;
+    const long long base = (long long)blockIdx.x * (SCAN_THREADS * SCAN_ITEMS) + (long long)threadIdx.x * SCAN_ITEMS;
     int v[SCAN_ITEMS];
     int s = 0;
+    scan_load<SCAN_ITEMS>(in, base, n, v);
 #pragma unroll
-    for (int k = 0; k < SCAN_ITEMS; ++k) {
-        v[k] = base + k < n ? in[base + k] : 0;
-        s += v[k];
-    }
+    for (int k = 0; k < SCAN_ITEMS; ++k) s += v[k];
     int total;
-    int ex = block_exclusive_scan(s, ws, total) + offset;
-#pragma unroll
-    for (int k = 0; k < SCAN_ITEMS; ++k) {
-        if (base + k < n) {
-            out[base + k] = ex;
-            if (zero) zero[base + k] = 0;
-        }
-        ex += v[k];
-    }
+    const int ex = block_exclusive_scan(s, ws, total) + offset;
+    scan_finish<SCAN_ITEMS>(out, zero, base, n, v, ex);
     if (blockIdx.x == nblocks - 1 && threadIdx.x == 0) *grand_total = offset + total;
 }
 
@@ -2681,15 +2736,35 @@ cudaError_t launch_reset_energy(float4* force, float4* vel, float4* vold, int n,
     return cudaGetLastError();
 }
 
-long long scan_block_count(long long n) { return (n + SCAN_TILE - 1) / SCAN_TILE; }
+long long scan_block_count(long long n) {
+    const long long tile = (long long)SCAN_THREADS * scan_items(n);
+    return (n + tile - 1) / tile;
+}
+
+template <int ITEMS>
+static void launch_scan(const int* in, long long n, int* out, int* block_sums, cudaStream_t s) {
+    const unsigned nblk = (unsigned)scan_block_count(n);
+    k_scan_partials<ITEMS><<<nblk, SCAN_THREADS, 0, s>>>(in, n, block_sums, nullptr);
+    k_scan_sums<<<1, SCAN_THREADS, 0, s>>>(block_sums, (int)nblk, out + n, nullptr);
+    k_scan_apply<ITEMS><<<nblk, SCAN_THREADS, 0, s>>>(in, n, block_sums, out, nullptr, nullptr);
+}
 
 cudaError_t launch_exclusive_scan(const int* in, long long n, int* out, int* block_sums, cudaStream_t s) {
     if (n <= 0) return cudaSuccess;
-    const long long nblk = scan_block_count(n);
-    launch_next(k_scan_partials, nblk, SCAN_THREADS, 0, s, in, n, block_sums, nullptr);
-    k_scan_sums<<<1, SCAN_THREADS, 0, s>>>(block_sums, (int)nblk, out + n, nullptr);
-    k_scan_apply<<<(unsigned)nblk, SCAN_THREADS, 0, s>>>(in, n, block_sums, out, nullptr, nullptr);
+    if (scan_items(n) == 8)
+        launch_scan<8>(in, n, out, block_sums, s);
+    else
+        launch_scan<2>(in, n, out, block_sums, s);
     return cudaGetLastError();
+}
+
+/* The rebuild's scan of the cell counts, as part of the step sequence. */
+template <int ITEMS>
+static void launch_cell_scan(const RebuildArgs& R, long long ncells, int* block_sums, cudaStream_t s) {
+    const unsigned nblk = (unsigned)scan_block_count(ncells);
+    launch_next(k_scan_partials<ITEMS>, nblk, SCAN_THREADS, 0, s, R.cell_count, ncells, block_sums, R.gate);
+    launch_next(k_scan_apply_direct<ITEMS>, nblk, SCAN_THREADS, 0, s, R.cell_count, ncells, block_sums, (int)nblk,
+                R.cell_start, R.cell_start + ncells, R.gate, R.cell_fill);
 }
 
 /* Largest context whose bead-by-bead build takes four lanes per bead: below
@@ -2716,13 +2791,16 @@ cudaError_t launch_rebuild(const RebuildArgs& R, int ntiles, int block, int nb, 
        k_cells, so only the cell counts need a pass of their own */
     launch_next(k_fill_int, fill_blocks, 256, 0, s, R.cell_count, ncells, 0, R.gate);
     if (ntiles > 0) launch_next(k_cells, ntiles, block, 0, s, R);
-    const long long nblk = scan_block_count(ncells);
-    launch_next(k_scan_partials, nblk, SCAN_THREADS, 0, s, R.cell_count, ncells, scan_block_sums, R.gate);
-    launch_next(k_scan_apply_direct, nblk, SCAN_THREADS, 0, s, R.cell_count, ncells, scan_block_sums, (int)nblk,
-                                                                 R.cell_start, R.cell_start + ncells, R.gate,
-                                                                 R.cell_fill);
+    if (scan_items(ncells) == 8)
+        launch_cell_scan<8>(R, ncells, scan_block_sums, s);
+    else
+        launch_cell_scan<2>(R, ncells, scan_block_sums, s);
     if (nb > 0) launch_next(k_scatter, (nb + 255) / 256, 256, 0, s, R, nb);
-    launch_next(k_cell_sort, (unsigned)((ncells + 255) / 256), 256, 0, s, R, (int)ncells);
+    /* 10 cells per bead (64 batched networks): 59 us against 210 */
+    if (nb > 0 && ncells >= SCAN_SMALL && ncells >= 4ll * nb)
+        launch_next(k_cell_sort_sparse, (nb + 255) / 256, 256, 0, s, R, nb, ncells);
+    else
+        launch_next(k_cell_sort, (unsigned)((ncells + 255) / 256), 256, 0, s, R, (int)ncells);
     if (R.bricks) {
         if (R.nbricks > 0) launch_next(k_lists_brick, R.nbricks, kBrickThreads, 0, s, R, R.bricks);
     } else if (nb > 0 && R.list_lanes == 8) {

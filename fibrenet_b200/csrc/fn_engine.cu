@@ -905,8 +905,8 @@ fn::StepArgs step_args(fn_ctx* c, bool pingpong) {
     A.ch_status = c->ch_status.p;
     A.nb = (int)c->nb;
     A.wide = c->wide ? 1 : 0;
-    A.uniform = c->uniform ? 1 : 0;
-    if (c->uniform) {
+    A.uniform = c->uniform;
+    if (c->uniform != fn::FN_CONST_NONE) {
         A.net0 = c->nets_h[0];
         A.pair0 = c->pairs_h[0];
     }
@@ -931,8 +931,8 @@ fn::RebuildArgs rebuild_args(fn_ctx* c) {
     R.cell_beads = c->cell_beads.p;
     R.cell_raw = c->cell_raw.p;
     R.cell_pos = c->cell_pos.p;
-    R.uniform = c->uniform ? 1 : 0;
-    if (c->uniform) {
+    R.uniform = c->uniform;
+    if (c->uniform != fn::FN_CONST_NONE) {
         R.net0 = c->nets_h[0];
         R.pair0 = c->pairs_h[0];
     }
@@ -1371,11 +1371,11 @@ static void set_totals(fn_ctx* c, long long nb, long long ns, long long na, long
     c->ns = ns;
     c->na = na;
     c->ncells = ncells;
-    /* one network whose bead types all meet by the same law: its constants
-       and that law travel as kernel parameters */
-    c->uniform = c->n_nets == 1 && !c->pairs_h.empty();
+    /* networks whose bead types all meet by the same law: that law, and the
+       constants of a single network, travel as kernel parameters */
+    c->uniform = c->pairs_h.empty() ? fn::FN_CONST_NONE : c->n_nets == 1 ? fn::FN_CONST_ALL : fn::FN_CONST_LAW;
     for (const FnPair& P : c->pairs_h)
-        if (std::memcmp(&P, &c->pairs_h[0], sizeof P) != 0) c->uniform = false;
+        if (std::memcmp(&P, &c->pairs_h[0], sizeof P) != 0) c->uniform = fn::FN_CONST_NONE;
     c->list_stride = (int)((nb + 31) / 32 * 32);
     c->grid_update_freq = c->info[0].grid_update_freq;
 }

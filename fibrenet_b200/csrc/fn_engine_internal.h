@@ -68,7 +68,7 @@ struct fn_ctx {
     std::vector<float4> sp_par_h;  // upload order (springs are not renumbered)
     std::vector<float2> an_par_h;
     bool damp = false;
-    bool uniform = false; /* one network, one pair law for all bead types */
+    int uniform = 0; /* fn::FN_CONST_*: one pair law for all bead types; one network */
     int grid_update_freq = 8;
 
     DevBuf<double4> pos[2], img[2];

@@ -614,6 +614,13 @@ __device__ __forceinline__ int block_scan_any(int v, int* warp_sums, int& total)
     return r;
 }
 
+/* A network's constants into shared memory, by the block's first threads. */
+__device__ __forceinline__ void copy_net(const FnNet* __restrict__ from, FnNet* to) {
+    static_assert(sizeof(FnNet) % 8 == 0 && sizeof(FnNet) / 8 <= 64, "one word per thread");
+    if (threadIdx.x < sizeof(FnNet) / 8)
+        reinterpret_cast<long long*>(to)[threadIdx.x] = reinterpret_cast<const long long*>(from)[threadIdx.x];
+}
+
 /* The spring from a bead to the next one, (x, y, z) apart (kernel.cl:377-424):
    their distance l and its inverse, the force on the bead, and the bead's
    status after the step. */
@@ -671,10 +678,11 @@ __device__ __forceinline__ void chain_gather(const double* f, const double* o, d
    records' direction is not read.  An angle takes its arms' lengths and
    their inverses from the springs' threads.  FORCES_ONLY evaluates the
    selected terms alone (no base force, no kick or drift, no status change).
-   UNIFORM reads the network's constants and its one pair law from the kernel
-   parameters, i.e. as constant operands, instead of loading them for every
-   contact (1M-bead tensile step 108 us against 120 with them loaded); contexts
-   with several networks or laws take the other form.
+   CONSTS says what comes from the kernel parameters, as constant operands,
+   instead of being loaded for every contact: the network's constants and its
+   one pair law (1M-bead tensile step 108 us against 120 with them loaded), the
+   law alone (several networks that share it), or nothing; a network's
+   constants then lie in shared memory.
    Bound by instruction issue and the latency of dependent loads and FP64
    chains, not by DRAM (229 MB per 1M-bead step).  Sharing the roots' seeds
    and the arms' lengths took it from 71.7M to 56.5M warp instructions: 130 to
@@ -682,7 +690,7 @@ __device__ __forceinline__ void chain_gather(const double* f, const double* o, d
    to 20 us at 111k beads (one wave of blocks).  At most 256 threads per block
    and 4 such blocks per SM, i.e. 64 registers: both resident warps and the
    registers that keep the next list index in flight hide the loads' latency. */
-template <bool DAMP, bool FORCES_ONLY, bool UNIFORM>
+template <bool DAMP, bool FORCES_ONLY, int CONSTS>
 __global__ void __launch_bounds__(kChainMaxBlock, 4) k_step_chain(const __grid_constant__ StepArgs A, int flags) {
     extern __shared__ __align__(32) unsigned char smem_raw[];
     const FnTile tile = A.tiles[blockIdx.x];
@@ -694,6 +702,9 @@ __global__ void __launch_bounds__(kChainMaxBlock, 4) k_step_chain(const __grid_c
     double* s_spf = reinterpret_cast<double*>(smem_raw + L.spf);
     double* s_ang = reinterpret_cast<double*>(smem_raw + L.ang);
     unsigned char* s_ok = smem_raw + L.ok;
+    __shared__ FnNet s_net;
+    if (CONSTS != FN_CONST_ALL) copy_net(A.nets + tile.net, &s_net);
+    const FnNet& N = CONSTS == FN_CONST_ALL ? A.net0 : s_net; /* past the first barrier */
 
     /* tiles and flags are written by no kernel of the step sequence; loading the
        bonds' records here too gains 2 % on 480 beads and costs 1.5 % on the
@@ -764,7 +775,6 @@ __global__ void __launch_bounds__(kChainMaxBlock, 4) k_step_chain(const __grid_c
     /* a block that stages this bead as halo may see the old status or the
        new one: a bond that dies in this step acts in neither case */
     if (!FORCES_ONLY && active && st != st0) A.ch_status[i] = (unsigned char)st;
-    const FnNet& N = UNIFORM ? A.net0 : A.nets[tile.net];
     double4 p = make_double4(0.0, 0.0, 0.0, 0.0);
     double Fx = 0.0, Fy = 0.0, Fz = 0.0;
     int nc = 0;
@@ -794,7 +804,7 @@ __global__ void __launch_bounds__(kChainMaxBlock, 4) k_step_chain(const __grid_c
         double4* s_pos = reinterpret_cast<double4*>(smem_raw + L.pos) + (tid & ~31);
         if (active) s_pos[lane] = p;
         auto contact = [&](double4 a, double4 b, double& Rx, double& Ry, double& Rz) {
-            return UNIFORM ? contact_force(N, A.pair0, a, b, Rx, Ry, Rz) : contact_eval(N, A.pairs, a, b, Rx, Ry, Rz);
+            return CONSTS != FN_CONST_NONE ? contact_force(N, A.pair0, a, b, Rx, Ry, Rz) : contact_eval(N, A.pairs, a, b, Rx, Ry, Rz);
         };
         /* direct phase: every lane first evaluates the leading KD items of its
            own list, one list row per iteration (coalesced loads, no window
@@ -923,7 +933,7 @@ __device__ __forceinline__ void wide_barrier() {
     asm volatile("barrier.cta.sync 2, %0;" ::"n"(kWideThreads) : "memory");
 }
 
-template <bool DAMP, bool UNIFORM>
+template <bool DAMP, int CONSTS>
 __global__ void __launch_bounds__(kWideThreads, 6) k_step_wide(const __grid_constant__ StepArgs A, int flags, int parts,
                                                                int width) {
     __shared__ double s_img[3 * 32], s_spf[3 * 33], s_ang[6 * 33];
@@ -934,7 +944,12 @@ __global__ void __launch_bounds__(kWideThreads, 6) k_step_wide(const __grid_cons
     const int begin = tile.begin + (blockIdx.x % parts) * width;
     const int n = min(tile.end - begin, width); /* may be <= 0: nothing to do */
     const int tid = threadIdx.x;
-    const FnNet& N = UNIFORM ? A.net0 : A.nets[tile.net];
+    __shared__ FnNet s_net;
+    if (CONSTS != FN_CONST_ALL) {
+        copy_net(A.nets + tile.net, &s_net);
+        __syncthreads();
+    }
+    const FnNet& N = CONSTS == FN_CONST_ALL ? A.net0 : s_net;
     await_previous();
     if (tid >= 32) {
         const int b = (tid - 32) >> 2, g = tid & 3;
@@ -961,7 +976,7 @@ __global__ void __launch_bounds__(kWideThreads, 6) k_step_wide(const __grid_cons
                     if (h == 1 && !two) break;
                     const double4 q = h == 0 ? q0 : q1;
                     double Rx = 0.0, Ry = 0.0, Rz = 0.0;
-                    const int acts = UNIFORM ? contact_force(N, A.pair0, p, q, Rx, Ry, Rz)
+                    const int acts = CONSTS != FN_CONST_NONE ? contact_force(N, A.pair0, p, q, Rx, Ry, Rz)
                                              : contact_eval(N, A.pairs, p, q, Rx, Ry, Rz);
                     const int at = k - k0 + 4 * h;
                     R[3 * at] = Rx;
@@ -2613,31 +2628,35 @@ cudaError_t launch_step_tiled(const StepArgs& A, int ntiles, int block, bool dam
     if (ntiles <= 0) return cudaSuccess;
     const size_t sm = step_tiled_smem(A.max_tile_sp, A.max_tile_an);
     const int flags = step_flags(do_drift, store_v);
-    if (damp && A.uniform)
+    const bool all = A.uniform == FN_CONST_ALL;
+    if (damp && all)
         launch_next(k_step_tiled<true, true>, ntiles, block, sm, s, A, flags);
     else if (damp)
         launch_next(k_step_tiled<true, false>, ntiles, block, sm, s, A, flags);
-    else if (A.uniform)
+    else if (all)
         launch_next(k_step_tiled<false, true>, ntiles, block, sm, s, A, flags);
     else
         launch_next(k_step_tiled<false, false>, ntiles, block, sm, s, A, flags);
     return cudaGetLastError();
 }
 
-template <bool DAMP, bool FO, bool UNI>
+template <bool DAMP, bool FO, int CONSTS>
 static cudaError_t set_chain_smem(size_t bytes) {
-    return cudaFuncSetAttribute(k_step_chain<DAMP, FO, UNI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    return cudaFuncSetAttribute(k_step_chain<DAMP, FO, CONSTS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)bytes);
 }
 
 cudaError_t prepare_step_chain(size_t bytes) {
     static size_t done[64] = {};
     if (!raise_limit(done, bytes)) return cudaSuccess;
     cudaError_t e;
-    if ((e = set_chain_smem<true, false, false>(bytes))) return e;
-    if ((e = set_chain_smem<true, false, true>(bytes))) return e;
-    if ((e = set_chain_smem<false, false, false>(bytes))) return e;
-    if ((e = set_chain_smem<false, false, true>(bytes))) return e;
-    return set_chain_smem<false, true, false>(bytes);
+    if ((e = set_chain_smem<true, false, FN_CONST_NONE>(bytes))) return e;
+    if ((e = set_chain_smem<true, false, FN_CONST_LAW>(bytes))) return e;
+    if ((e = set_chain_smem<true, false, FN_CONST_ALL>(bytes))) return e;
+    if ((e = set_chain_smem<false, false, FN_CONST_NONE>(bytes))) return e;
+    if ((e = set_chain_smem<false, false, FN_CONST_LAW>(bytes))) return e;
+    if ((e = set_chain_smem<false, false, FN_CONST_ALL>(bytes))) return e;
+    return set_chain_smem<false, true, FN_CONST_NONE>(bytes);
 }
 
 cudaError_t launch_step_chain(const StepArgs& A, int ntiles, int block, bool damp, bool do_drift,
@@ -2647,24 +2666,22 @@ cudaError_t launch_step_chain(const StepArgs& A, int ntiles, int block, bool dam
     const int flags = step_flags(do_drift, store_v);
     if (A.wide) {
         const int parts = (block - 4 + kWideBeads - 1) / kWideBeads, width = (block - 4 + parts - 1) / parts;
-        if (damp && A.uniform)
-            launch_next(k_step_wide<true, true>, ntiles * parts, kWideThreads, 0, s, A, flags, parts, width);
-        else if (damp)
-            launch_next(k_step_wide<true, false>, ntiles * parts, kWideThreads, 0, s, A, flags, parts, width);
-        else if (A.uniform)
-            launch_next(k_step_wide<false, true>, ntiles * parts, kWideThreads, 0, s, A, flags, parts, width);
+        auto go = [&](auto kernel) { launch_next(kernel, ntiles * parts, kWideThreads, 0, s, A, flags, parts, width); };
+        if (A.uniform == FN_CONST_ALL)
+            damp ? go(k_step_wide<true, FN_CONST_ALL>) : go(k_step_wide<false, FN_CONST_ALL>);
+        else if (A.uniform == FN_CONST_LAW)
+            damp ? go(k_step_wide<true, FN_CONST_LAW>) : go(k_step_wide<false, FN_CONST_LAW>);
         else
-            launch_next(k_step_wide<false, false>, ntiles * parts, kWideThreads, 0, s, A, flags, parts, width);
+            damp ? go(k_step_wide<true, FN_CONST_NONE>) : go(k_step_wide<false, FN_CONST_NONE>);
         return cudaGetLastError();
     }
-    if (damp && A.uniform)
-        launch_next(k_step_chain<true, false, true>, ntiles, block, sm, s, A, flags);
-    else if (damp)
-        launch_next(k_step_chain<true, false, false>, ntiles, block, sm, s, A, flags);
-    else if (A.uniform)
-        launch_next(k_step_chain<false, false, true>, ntiles, block, sm, s, A, flags);
+    auto go = [&](auto kernel) { launch_next(kernel, ntiles, block, sm, s, A, flags); };
+    if (A.uniform == FN_CONST_ALL)
+        damp ? go(k_step_chain<true, false, FN_CONST_ALL>) : go(k_step_chain<false, false, FN_CONST_ALL>);
+    else if (A.uniform == FN_CONST_LAW)
+        damp ? go(k_step_chain<true, false, FN_CONST_LAW>) : go(k_step_chain<false, false, FN_CONST_LAW>);
     else
-        launch_next(k_step_chain<false, false, false>, ntiles, block, sm, s, A, flags);
+        damp ? go(k_step_chain<true, false, FN_CONST_NONE>) : go(k_step_chain<false, false, FN_CONST_NONE>);
     return cudaGetLastError();
 }
 
@@ -2710,7 +2727,7 @@ cudaError_t launch_step_staged(const StepArgs& A, int ntiles, int block, bool da
 
 cudaError_t launch_forces_chain(const StepArgs& A, int ntiles, int block, int terms, cudaStream_t s) {
     if (ntiles <= 0) return cudaSuccess;
-    launch_next(k_step_chain<false, true, false>, ntiles, block, step_chain_smem(block), s, A, terms);
+    launch_next(k_step_chain<false, true, FN_CONST_NONE>, ntiles, block, step_chain_smem(block), s, A, terms);
     return cudaGetLastError();
 }
 
@@ -2778,7 +2795,7 @@ constexpr int kGroupedBeads = 200000;
 template <int G>
 static void launch_lists_group(const RebuildArgs& R, int nb, long long ncells, cudaStream_t s) {
     constexpr int PER = 128 / G;
-    if (R.uniform)
+    if (R.uniform == FN_CONST_ALL)
         launch_next(k_lists_group<G, true>, (nb + PER - 1) / PER, 128, 0, s, R, ncells);
     else
         launch_next(k_lists_group<G, false>, (nb + PER - 1) / PER, 128, 0, s, R, ncells);
@@ -2808,7 +2825,7 @@ cudaError_t launch_rebuild(const RebuildArgs& R, int ntiles, int block, int nb, 
     } else if (nb > 0 && nb <= kGroupedBeads) {
         launch_lists_group<4>(R, nb, ncells, s);
     } else if (nb > 0) {
-        if (R.uniform)
+        if (R.uniform == FN_CONST_ALL)
             launch_next(k_lists<true>, (nb + 127) / 128, 128, 0, s, R, ncells);
         else
             launch_next(k_lists<false>, (nb + 127) / 128, 128, 0, s, R, ncells);

@@ -11,6 +11,10 @@
 
 namespace fn {
 
+/* What the kernels get by value: nothing, the one pair law that all beads of
+   all networks meet by, or that law and the constants of the only network. */
+enum { FN_CONST_NONE = 0, FN_CONST_LAW = 1, FN_CONST_ALL = 2 };
+
 struct StepArgs {
     const FnTile* tiles;
     const FnNet* nets;
@@ -68,8 +72,7 @@ struct StepArgs {
     long long csr_region;
     const int* tile_items;
     int chunk; /* contact items staged per round (a multiple of the block size) */
-    /* one network with one pair law for all bead types: both by value, so
-       that the chain kernel reads them as constants */
+    /* FN_CONST_*: by value, so that the kernels read them as constants */
     int uniform;
     FnNet net0;
     FnPair pair0;
@@ -237,8 +240,7 @@ struct RebuildArgs {
     int* csr;
     long long csr_region;
     int* tile_items;
-    /* one network with one pair law for all bead types: both by value */
-    int uniform;
+    int uniform; /* FN_CONST_* */
     FnNet net0;
     FnPair pair0;
 };

@@ -1970,6 +1970,19 @@ FN_API int fn_device_view(fn_ctx* c, int field, fn_view* out) {
     FN_CATCH(c)
 }
 
+/* Touches every page of a buffer that a copy is about to fill, on host threads:
+   the pages of a large fresh allocation are mapped one fault after the other
+   otherwise, inside the copy (76 MB: 17.7 ms, 4.4 with the pages present),
+   while here the device is still busy with what the copy waits for.  Bytes
+   keep their values. */
+static void touch_pages(void* buffer, size_t bytes) {
+    constexpr size_t kUnit = 128, kPage = 4096;
+    volatile char* p = static_cast<volatile char*>(buffer);
+    fnh::parallel_for((long long)(bytes / kUnit), [p](long long b, long long e) {
+        for (size_t at = (size_t)b * kUnit; at < (size_t)e * kUnit; at += kPage) p[at] = p[at];
+    });
+}
+
 FN_API int fn_download(fn_ctx* c, int field, double* host) {
     FN_TRY
     fnh::NvtxRange nvtx_range_("fn_download");
@@ -1996,6 +2009,7 @@ FN_API int fn_download(fn_ctx* c, int field, double* host) {
         if (!b) return fail(c, FN_ERR_ARG, "fn_download: unknown field");
         CK(fn::launch_export_xyz(b->p, c->inv_d.p, (int)nb, c->export_xyz.p, c->stream));
     }
+    if (sizeof(double) * 3 * nb >= ((size_t)16 << 20)) touch_pages(host, sizeof(double) * 3 * nb);
     CK(cudaMemcpyAsync(host, c->export_xyz.p, sizeof(double) * 3 * nb, cudaMemcpyDeviceToHost, c->stream));
     CK(cudaStreamSynchronize(c->stream));
     return FN_OK;

@@ -38,6 +38,7 @@
 #include "fn_detmath.h"
 #include "fn_device.cuh"
 #include "fn_engine_internal.h"
+#include "fn_rounded.cuh"
 
 namespace fn {
 
@@ -60,6 +61,25 @@ __device__ __forceinline__ Dual dsqrt(Dual a) {
     return {r, r > 0.0 ? a.d / (2.0 * r) : 0.0};
 }
 
+/* A root that later divides: its value, tangent and 1/value, which the
+   quotients by it share (the bits of a plain division, fn_rounded.cuh). */
+struct DualRoot {
+    double v, d, inv;
+};
+__device__ __forceinline__ double over(double a, double b, double inv) {
+    return inv > 0.0 ? quotient(a, b, inv) : a / b;
+}
+__device__ __forceinline__ DualRoot droot(Dual a) {
+    double r, ir;
+    root_and_inverse(a.v, r, ir);
+    return {r, r > 0.0 ? over(a.d, 2.0 * r, 0.5 * ir) : 0.0, ir};
+}
+__device__ __forceinline__ Dual operator/(Dual a, DualRoot b) {
+    const double q = over(a.v, b.v, b.inv);
+    return {q, over(a.d - q * b.d, b.v, b.inv)};
+}
+__device__ __forceinline__ Dual value(DualRoot a) { return {a.v, a.d}; }
+
 /* The angle force of kernel.cl:291-348 at unit stiffness, with tangents:
    t1..t3 positions of b1..b3 with tangent directions w1..w3.  Returns pa (on
    b1) and pc (on b3) as duals; the force scales linearly with the stiffness.
@@ -72,9 +92,9 @@ __device__ void angle_dual(const double* t1, const double* t2, const double* t3,
         bc[a] = {t3[a] - t2[a], (double)w3[a] - (double)w2[a]};
         cb[a] = bc[a] * -1.0;
     }
-    const Dual l_ba = dsqrt(ba[0] * ba[0] + ba[1] * ba[1] + ba[2] * ba[2]);
-    const Dual l_bc = dsqrt(bc[0] * bc[0] + bc[1] * bc[1] + bc[2] * bc[2]);
-    Dual dotp = (ba[0] * bc[0] + ba[1] * bc[1] + ba[2] * bc[2]) / (l_ba * l_bc);
+    const DualRoot l_ba = droot(ba[0] * ba[0] + ba[1] * ba[1] + ba[2] * ba[2]);
+    const DualRoot l_bc = droot(bc[0] * bc[0] + bc[1] * bc[1] + bc[2] * bc[2]);
+    Dual dotp = (ba[0] * bc[0] + ba[1] * bc[1] + ba[2] * bc[2]) / (value(l_ba) * value(l_bc));
     if (dotp.v < -1.0) dotp = dl(-0.999999);
     if (dotp.v > 1.0) dotp = dl(0.999999);
     const double s = 1.0 - dotp.v * dotp.v;
@@ -88,13 +108,13 @@ __device__ void angle_dual(const double* t1, const double* t2, const double* t3,
     pa[0] = ba[1] * tz - ba[2] * ty;
     pa[1] = ba[2] * tx - ba[0] * tz;
     pa[2] = ba[0] * ty - ba[1] * tx;
-    Dual ln = dsqrt(pa[0] * pa[0] + pa[1] * pa[1] + pa[2] * pa[2]);
+    DualRoot ln = droot(pa[0] * pa[0] + pa[1] * pa[1] + pa[2] * pa[2]);
     Dual sc = ln.v != 0.0 ? fa / ln : dl(0.0);
     for (int a = 0; a < 3; ++a) pa[a] = pa[a] * sc;
     pc[0] = cb[1] * tz - cb[2] * ty;
     pc[1] = cb[2] * tx - cb[0] * tz;
     pc[2] = cb[0] * ty - cb[1] * tx;
-    ln = dsqrt(pc[0] * pc[0] + pc[1] * pc[1] + pc[2] * pc[2]);
+    ln = droot(pc[0] * pc[0] + pc[1] * pc[1] + pc[2] * pc[2]);
     sc = ln.v != 0.0 ? fc / ln : dl(0.0);
     for (int a = 0; a < 3; ++a) pc[a] = pc[a] * sc;
 }
@@ -128,8 +148,8 @@ __device__ void angle_dual_straight(const double* t1, const double* t2, const do
         for (int a = 0; a < 3; ++a) pa[a] = pc[a] = dl(0.0);
         return;
     }
-    const Dual l_ba = dsqrt(ba[0] * ba[0] + ba[1] * ba[1] + ba[2] * ba[2]);
-    const Dual l_bc = dsqrt(bc[0] * bc[0] + bc[1] * bc[1] + bc[2] * bc[2]);
+    const DualRoot l_ba = droot(ba[0] * ba[0] + ba[1] * ba[1] + ba[2] * ba[2]);
+    const DualRoot l_bc = droot(bc[0] * bc[0] + bc[1] * bc[1] + bc[2] * bc[2]);
     Dual u[3], w[3];
     for (int a = 0; a < 3; ++a) {
         u[a] = ba[a] / l_ba;
@@ -157,11 +177,10 @@ __device__ void angle_dual_straight(const double* t1, const double* t2, const do
 }
 
 /* Tangent of a central pair force f(r) r_hat along dr: (f/r)(dr - r_hat
-   (r_hat.dr)) + f'(r) r_hat (r_hat.dr). */
-__device__ __forceinline__ void central_tangent(double rx, double ry, double rz, double r, double f,
+   (r_hat.dr)) + f'(r) r_hat (r_hat.dr), with ir = 1/r (0 for r = 0). */
+__device__ __forceinline__ void central_tangent(double rx, double ry, double rz, double ir, double f,
                                                 double fp, double dx, double dy, double dz, double& tx,
                                                 double& ty, double& tz) {
-    const double ir = r > 0.0 ? 1.0 / r : 0.0;
     const double ux = rx * ir, uy = ry * ir, uz = rz * ir;
     const double ud = ux * dx + uy * dy + uz * dz;
     const double fr = f * ir;
@@ -173,15 +192,16 @@ __device__ __forceinline__ void central_tangent(double rx, double ry, double rz,
 /* Radial contact force f(r) and its derivative for one listed pair, under
    the same acting conditions as the step's contact term. */
 __device__ __forceinline__ int contact_f(const FnNet& N, const FnPair* __restrict__ pairs, double4 pi,
-                                         double4 pj, double r2, double& f, double& fp) {
+                                         double4 pj, double r2, double& f, double& fp, double& ir) {
     const FnPair* P = pairs + N.pair_base + getadress(w_type(pi.w), w_type(pj.w), N.types_num);
     const int kind = P->kind;
-    const double r = sqrt(r2);
+    double r;
+    root_and_inverse(r2, r, ir);
     if (kind == 1) {
         if (!(r2 < N.cutoff_sq) || !(r < P->c[2])) return 0;
         const double s2 = P->c[0] * P->c[0], eps = P->c[1];
         const double s6 = s2 * s2 * s2, s12 = s6 * s6;
-        const double ir = 1.0 / r;
+        if (r == 0.0) ir = 1.0 / r;
         const double ir2 = ir * ir, ir4 = ir2 * ir2, ir8 = ir4 * ir4;
         const double ir14 = ir8 * ir4 * ir2;
         f = 48.0 * eps * s12 * ir14 - 24.0 * eps * s6 * ir8 - P->c[3];
@@ -283,14 +303,15 @@ __global__ void __launch_bounds__(256) k_adj_bonds(const AdjArgs A) {
             const float4 par = A.sp_par[s];
             const float4 w1 = A.fbar[e.x], w2 = A.fbar[e.y];
             const double rx = a.x - b.x, ry = a.y - b.y, rz = a.z - b.z;
-            const double L = sqrt(rx * rx + ry * ry + rz * rz);
+            double L, iL;
+            root_and_inverse(rx * rx + ry * ry + rz * rz, L, iL);
             const double dx = (double)w1.x - (double)w2.x, dy = (double)w1.y - (double)w2.y,
                          dz = (double)w1.z - (double)w2.z;
             const double k = par.y, rest = par.x;
             double tx, ty, tz;
-            central_tangent(rx, ry, rz, L, k * (rest - L), -k, dx, dy, dz, tx, ty, tz);
+            central_tangent(rx, ry, rz, iL, k * (rest - L), -k, dx, dy, dz, tx, ty, tz);
             out = make_float4((float)tx, (float)ty, (float)tz, 0.f);
-            const double ud = L > 0.0 ? (rx * dx + ry * dy + rz * dz) / L : 0.0;
+            const double ud = L > 0.0 ? over(rx * dx + ry * dy + rz * dz, L, iL) : 0.0;
             double2 g = A.g_spring[s];
             g.x += (rest - L) * ud;
             g.y += k * ud;
@@ -395,17 +416,21 @@ __global__ void __launch_bounds__(512) k_adj_beads(const AdjArgs A) {
     }
     int n = A.list_count[i];
     if (n > A.list_cap) n = A.list_cap;
+    const int* row = A.list + i;
+    int jn = *row;
     for (int k = 0; k < n; ++k) {
-        const int j = A.list[(size_t)k * A.list_stride + i];
+        const int j = jn;
+        if (k + 1 < A.list_cap) row += A.list_stride;
+        jn = *row; /* the next index, loaded one item ahead */
         const double4 pj = A.pos[j];
+        const float4 wj = A.fbar[j];
         double rx = p.x - pj.x, ry = p.y - pj.y, rz = p.z - pj.z;
         double r2 = rx * rx + ry * ry + rz * rz;
         r2 = min_image(N, rx, ry, rz, r2, N.force_mi);
-        double f, fp;
-        if (!contact_f(N, A.pairs, p, pj, r2, f, fp)) continue;
-        const float4 wj = A.fbar[j];
+        double f, fp, ir;
+        if (!contact_f(N, A.pairs, p, pj, r2, f, fp, ir)) continue;
         double tx, ty, tz;
-        central_tangent(rx, ry, rz, sqrt(r2), f, fp, (double)wi.x - (double)wj.x,
+        central_tangent(rx, ry, rz, ir, f, fp, (double)wi.x - (double)wj.x,
                         (double)wi.y - (double)wj.y, (double)wi.z - (double)wj.z, tx, ty, tz);
         jx += tx;
         jy += ty;

@@ -81,3 +81,28 @@ def test_distances_outside_the_shared_seed_range(oracle_built, law, gap):
         m.pos[1] = m.img[1] = (0.6, 0.0, 0.0)
         m.pos[2] = m.img[2] = (0.0, 0.7, gap)
     equal_to_mirror(m, [2])
+
+
+# both chain kernels that read networks' settings from tables and the one pair
+# law from the kernel parameters: by default the small-context form, with a
+# block size one thread per bead
+@pytest.mark.parametrize("block", [0, 64])
+@pytest.mark.parametrize("law", sorted(LAWS))
+def test_networks_of_one_law(oracle_built, law, block):
+    from fibrenet_b200.native import Simulation
+    ms = [network(law, True, beads, fibres) for beads, fibres in ((33, 3), (1, 5), (60, 2))]
+    for k, m in enumerate(ms):
+        m.settings.damping = 0.1 * k
+    with Simulation(ms, reorder=False, list_capacity=64, block_size=block) as s:
+        s.step(1)
+        s.step(11)
+        got = {f: s.get(f) for f in FIELDS}
+    first = 0
+    for m in ms:
+        o = po.OracleSim(m, po.MODE_MIRROR, cell_cap=64, list_cap=64)
+        o.run(1)
+        o.run(11)
+        n = len(o.get("pos"))
+        for f in FIELDS:
+            np.testing.assert_array_equal(got[f][first:first + n], o.get(f), err_msg=f)
+        first += n

@@ -1974,12 +1974,19 @@ FN_API int fn_device_view(fn_ctx* c, int field, fn_view* out) {
    the pages of a large fresh allocation are mapped one fault after the other
    otherwise, inside the copy (76 MB: 17.7 ms, 4.4 with the pages present),
    while here the device is still busy with what the copy waits for.  Bytes
-   keep their values. */
+   keep their values.  Only the caller's pageable memory: pinned pages are
+   there, and any other address is the copy's to take or refuse. */
 static void touch_pages(void* buffer, size_t bytes) {
+    cudaPointerAttributes at{};
+    if (cudaPointerGetAttributes(&at, buffer) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return;
+    }
+    if (at.type != cudaMemoryTypeUnregistered) return;
     constexpr size_t kUnit = 128, kPage = 4096;
     volatile char* p = static_cast<volatile char*>(buffer);
     fnh::parallel_for((long long)(bytes / kUnit), [p](long long b, long long e) {
-        for (size_t at = (size_t)b * kUnit; at < (size_t)e * kUnit; at += kPage) p[at] = p[at];
+        for (size_t o = (size_t)b * kUnit; o < (size_t)e * kUnit; o += kPage) p[o] = p[o];
     });
 }
 

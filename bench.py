@@ -43,7 +43,7 @@ METRIC = "bead-steps/s (tensile network, 1 B200 per replica)"
 UNIT = "bead-steps/s"
 WORKLOAD = "tensile_1M"
 OUTPUT_FREQ = 100  # the tensile test records reaction force / broken springs every 100 steps
-REBUILD_KERNELS = 6  # k_cells, two scan kernels, k_scatter, k_cell_sort, the list build
+REBUILD_KERNELS = 7  # clearing the cell counts, k_cells, two scan kernels, k_scatter, the cell sort, the list build
 
 
 def parse():

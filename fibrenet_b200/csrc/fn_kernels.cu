@@ -1931,7 +1931,8 @@ constexpr int kListKeep = 24;
    Bound by instruction issue (about 3,300 per warp, 60 % of the slots) and
    load latency.  The FP32 test from 16 bytes per candidate, with FP64 only
    where it cannot decide, took the rebuild of the 1M-bead tensile network
-   from 313 to 211 us and that of the 4M-bead mat from 1,340 to 943 us. */
+   from 313 to 211 us and that of the 4M-bead mat from 1,340 to 943 us (202
+   and 904 since its launches are chained and its scan reads wider). */
 template <bool UNIFORM>
 __global__ void __launch_bounds__(128, 8) k_lists(const __grid_constant__ RebuildArgs R, long long ncells) {
     await_previous();
@@ -2758,8 +2759,8 @@ static void launch_cell_scan(const RebuildArgs& R, long long ncells, int* block_
 }
 
 /* Largest context whose bead-by-bead build takes four lanes per bead: below
-   it one thread per bead leaves the SMs waiting for its loads (whole rebuild,
-   four lanes against one: 10k beads 38 against 42 us, 100k dense 60 against
+   it one thread per bead leaves the SMs waiting for its loads (whole rebuild
+   before its launches were chained, four lanes against one: 10k beads 38 against 42 us, 100k dense 60 against
    91, 111k tensile 68 against 66), above it the instructions of the scan and
    the ballots count (300k tensile 111 against 90, 1M 320 against 211). */
 constexpr int kGroupedBeads = 200000;

@@ -10,11 +10,11 @@ namespace fn {
 /* Programmatic dependent launch (launch_next): a kernel of the step sequence
    or of the adjoint sweep waits on the device for the kernel before it, all of
    its blocks and writes, before it touches anything that the kernels of its
-   chain write, and says when the next one's blocks may be placed.  The launch itself, 1.5 us and more between dependent
-   kernels of a stream, then runs beside the kernel before it.  Every thread of
-   every kernel that launch_next starts must wait, whatever it does next: one
-   that ended without waiting would let its successor run beside its
-   predecessor. */
+   chain write, and says when the next one's blocks may be placed.  The launch
+   itself, 1.5 us and more between dependent kernels of a stream, then runs
+   beside the kernel before it.  Every thread of every kernel that launch_next
+   starts must wait, whatever it does next: one that ended without waiting
+   would let its successor run beside its predecessor. */
 __device__ __forceinline__ void await_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void let_next_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 

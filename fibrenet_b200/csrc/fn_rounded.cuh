@@ -7,8 +7,8 @@
  * As separate operators each of them starts from a seed of its own, tests its
  * own range and branches to its own slow path; here one reciprocal square
  * root seeds them all and one range test covers them, so a Lennard-Jones
- * contact's root, reciprocal and two quotients are 18 multiply-adds and one
- * seed with no branch between them.
+ * contact's root, its reciprocal and two quotients are 24 multiplications and
+ * multiply-adds and one seed with no branch between them.
  *
  * The corrections are the classical ones for hardware with a fused
  * multiply-add (P. Markstein, "Computation of elementary functions on the
@@ -18,21 +18,24 @@
  * more fused operation adds it.  With u = 2^-52:
  *   root        y ~ 1/sqrt(d) to 0.75 u; s = d y; s + (d - s s) y/2 differs
  *               from the root by less than 3.4 u^2 before it is rounded;
- *   reciprocal  y ~ 1/b to 2 u; y + y (1 - b y) differs from 1/b by the
- *               square of y's error, below 4 u^2/b, and always from below;
+ *   reciprocal  y ~ 1/b to 2 u; r = y + y (1 - b y) differs from 1/b by less
+ *               than 4 u^2/b before it is rounded, so r is one of the two
+ *               doubles around 1/b; r + r (1 - b r) is then below 1/b by
+ *               b 2^-108 at most (b in [1, 2)), while the middle of two
+ *               doubles that lies below 1/b lies k 2^-106/b below it for a
+ *               whole k > 0.  b^2 < 4: no middle is between, the result is
+ *               rounded as 1/b is, but for b = 2 - u, where the two meet;
  *   quotient    with y = 1/b correctly rounded, q = a y, q + y (a - b q) is
  *               a/b correctly rounded (Markstein's theorem).
- * A root or a reciprocal can round differently from the operator only where
- * the exact value lies within those errors of the middle of two doubles: for
- * a root where d - m^2 is a multiple k 2^-107 of d's binade with |k| < 54, m
- * the middle; for a reciprocal where b m = 1 - k 2^-106, 0 < k <= 16.  All
- * such operands (3,235 mantissas, found by square roots modulo 2^54 and by
- * factoring 2^106 - k) and 9e9 random ones were compared with the operators:
- * every root and every quotient is the operator's, and so is every reciprocal
- * but those of a few dozen mantissas out of 2^52, which may come out one unit
- * in the last place apart.  The one of them that real inputs meet, 2^53 - 1
- * (squared distances a rounding below 1 or 4: straight fibres of unit
- * spacing), is corrected.
+ * A root can round differently from the operator only where d - m^2 is a
+ * multiple k 2^-107 of d's binade with |k| < 54, m the middle of two doubles.
+ * Those operands (found by square roots modulo 2^54), the mantissas whose
+ * reciprocals lie closest to a middle (the divisors of 2^106 - k, k <= 16),
+ * quotients next to a middle and random operands are compared with the IEEE
+ * operations by the GPU tests: every bit is the same.  (With one correction of
+ * the reciprocal instead of two, some dozens of mantissas came out one unit
+ * in the last place apart; the second costs 0.7 % of a run: 100 steps of the
+ * 1M-bead tensile network 15.05 -> 15.16 ms, 50 of 111k beads 1.62 -> 1.64.)
  */
 #ifndef FIBRENET_ROUNDED_CUH
 #define FIBRENET_ROUNDED_CUH
@@ -66,8 +69,9 @@ __device__ __forceinline__ double root_from(double d, double y) {
    one unit below the rounded reciprocal (Markstein's exception). */
 __device__ __forceinline__ double recip_from(double b, double y) {
     const double r = __fma_rn(__fma_rn(-b, y, 1.0), y, y);
+    const double s = __fma_rn(__fma_rn(-b, r, 1.0), r, r);
     const int ones = (__double2hiint(b) | (int)0xfff00000) & __double2loint(b);
-    return __hiloint2double(__double2hiint(r), __double2loint(r) | (ones == -1 ? 1 : 0));
+    return __hiloint2double(__double2hiint(s), __double2loint(s) | (ones == -1 ? 1 : 0));
 }
 
 /* a/b, y = 1/b correctly rounded */

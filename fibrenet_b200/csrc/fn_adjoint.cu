@@ -68,7 +68,7 @@ struct DualRoot {
     double v, d, inv;
 };
 __device__ __forceinline__ double over(double a, double b, double inv) {
-    return inv > 0.0 ? quotient(a, b, inv) : a / b;
+    return inv > 0.0 ? quotient_any(a, b, inv) : a / b;
 }
 __device__ __forceinline__ DualRoot droot(Dual a) {
     double r, ir;

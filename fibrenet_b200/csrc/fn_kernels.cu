@@ -114,13 +114,15 @@ __device__ __forceinline__ void angle_arms(double bax, double bay, double baz, d
     const double dot = bax * bcx + bay * bcy + baz * bcz;
     const double ll = l_ba * l_bc;
     const bool fast = fn_fast_range(ll);
+    /* |dot| <= ll up to rounding: finite, and where it is too small for the
+       quotient's residual the arc cosine does not see it */
     double dotp = fast ? quotient(dot, ll, recip_from(ll, il_ba * il_bc)) : dot / ll;
     if (dotp < -1.0) dotp = -0.999999;
     if (dotp > 1.0) dotp = 0.999999;
     const double angle = acos_rounded(dotp);
     const double magnitude = -2.0 * (double)par.y * (angle - (double)par.x);
-    const double fa = fast ? quotient(magnitude, l_ba, il_ba) : magnitude / l_ba;
-    const double fc = fast ? quotient(magnitude, l_bc, il_bc) : magnitude / l_bc;
+    const double fa = fast ? quotient_any(magnitude, l_ba, il_ba) : magnitude / l_ba;
+    const double fc = fast ? quotient_any(magnitude, l_bc, il_bc) : magnitude / l_bc;
     const double tx = bay * bcz - baz * bcy;
     const double ty = baz * bcx - bax * bcz;
     const double tz = bax * bcy - bay * bcx;

@@ -26,7 +26,8 @@
  *               whole k > 0.  b^2 < 4: no middle is between, the result is
  *               rounded as 1/b is, but for b = 2 - u, where the two meet;
  *   quotient    with y = 1/b correctly rounded, q = a y, q + y (a - b q) is
- *               a/b correctly rounded (Markstein's theorem).
+ *               a/b correctly rounded (Markstein's theorem; where a/b is next
+ *               to a middle, q is one of the two doubles around it).
  * A root can round differently from the operator only where d - m^2 is a
  * multiple k 2^-107 of d's binade with |k| < 54, m the middle of two doubles.
  * Those operands (found by square roots modulo 2^54), the mantissas whose
@@ -74,10 +75,21 @@ __device__ __forceinline__ double recip_from(double b, double y) {
     return __hiloint2double(__double2hiint(s), __double2loint(s) | (ones == -1 ? 1 : 0));
 }
 
-/* a/b, y = 1/b correctly rounded */
+/* a/b, y = 1/b correctly rounded, neither a nor a/b near the ends of the
+   normal range */
 __device__ __forceinline__ double quotient(double a, double b, double y) {
     const double q = __dmul_rn(a, y);
     return __fma_rn(__fma_rn(-b, q, a), y, q);
+}
+
+/* The same for any numerator, b a finite root above 0 (2^-537 .. 2^512).  In
+   [2^-400, 2^400) the residual is exact and the quotient normal; a zero, as
+   most tangents of an adjoint sweep's first steps are, keeps its sign; what is
+   left, infinities among it (whose residual is NaN), takes the operator. */
+__device__ __forceinline__ double quotient_any(double a, double b, double y) {
+    const unsigned h = (unsigned)__double2hiint(a) & 0x7fffffffu;
+    if (h - 0x26f00000u < 0x32000000u) return quotient(a, b, y);
+    return a == 0.0 ? __dmul_rn(a, y) : a / b;
 }
 
 /* l = sqrt(d) and il = 1/l as the operators give them (il = 0 for l = 0, as

@@ -11,7 +11,7 @@
 
 using namespace fn;
 
-enum { OP_ROOT = 0, OP_INVERSE_ROOT = 1, OP_PRODUCT_INVERSE = 2, OP_SQUARE_INVERSE = 3, OP_QUOTIENT = 4 };
+enum { OP_ROOT = 0, OP_INVERSE_ROOT = 1, OP_PRODUCT_INVERSE = 2, OP_SQUARE_INVERSE = 3, OP_QUOTIENT = 4, OP_QUOTIENT_ANY = 5 };
 
 static __global__ void k_rounded(int op, const double* a, const double* b, double* out, long long n) {
     const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
@@ -37,6 +37,9 @@ static __global__ void k_rounded(int op, const double* a, const double* b, doubl
         break;
     case OP_QUOTIENT: /* a / b */
         r = quotient(a[i], b[i], 1.0 / b[i]);
+        break;
+    case OP_QUOTIENT_ANY: /* a / b for any a, b a finite root above 0 */
+        r = quotient_any(a[i], b[i], 1.0 / b[i]);
         break;
     }
     out[i] = r;

@@ -14,7 +14,7 @@ pytestmark = pytest.mark.gpu
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 HERE = os.path.join(ROOT, "tests", "rounded")
 HEADER = os.path.join(ROOT, "fibrenet_b200", "csrc", "fn_rounded.cuh")
-OPS = OP_ROOT, OP_INVERSE_ROOT, OP_PRODUCT_INVERSE, OP_SQUARE_INVERSE, OP_QUOTIENT = range(5)
+OP_ROOT, OP_INVERSE_ROOT, OP_PRODUCT_INVERSE, OP_SQUARE_INVERSE, OP_QUOTIENT, OP_QUOTIENT_ANY = range(6)
 
 # 2^106 - k = product of the primes, k = 1 .. 16
 FACTORS = {
@@ -199,3 +199,18 @@ def test_quotient(run):
     a = np.concatenate([ha, -ha, 1.0 + rng.random(rb.size * 50), randoms(4_000_000, -200, 200, 9)])
     b = np.concatenate([hb, hb, np.repeat(rb, 50), randoms(4_000_000, -200, 200, 10)])
     same_bits(run(OP_QUOTIENT, a, b), a / b, a, b)
+
+
+def test_quotient_of_any_numerator(run):
+    """Zeros, infinities, NaN and numerators at the ends of the range of doubles
+    and of the fast sequence, over divisors as roots are."""
+    rng = np.random.default_rng(12)
+    tiny = np.array([5e-324, 3e-320, 2.0**-1022, 2.0**-970, np.finfo(float).max, 0.0, np.inf])
+    edges = around(np.ldexp(1.0, [-401, -400, -399, 399, 400, 401]), 2)
+    a = np.concatenate([tiny, edges, randoms(20_000, -1070, 1023, 13)])
+    a = np.concatenate([a, -a, [np.nan]])
+    b = np.concatenate([1.0 + rng.random(64), np.ldexp(1.0 + rng.random(64), rng.integers(-537, 511, 64)),
+                        hard_reciprocals()[::8], np.ldexp(1.0, [-537, -200, -1, 0, 1, 511])])
+    a, b = (np.ascontiguousarray(v).ravel() for v in np.meshgrid(a, b))
+    with np.errstate(over="ignore", under="ignore", invalid="ignore"):
+        same_bits(run(OP_QUOTIENT_ANY, a, b), a / b, a, b)

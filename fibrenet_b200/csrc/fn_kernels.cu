@@ -2900,6 +2900,7 @@ __device__ __forceinline__ double contact_energy(const FnNet& N, const FnPair* _
         const double rc = P->c[2], s2 = P->c[0] * P->c[0], eps = P->c[1];
         const double s6 = s2 * s2 * s2, s12 = s6 * s6;
         const double irc = 1.0 / rc;
+        if (r == 0.0) ir = 1.0 / r; /* the force terms take 0 there; the potential is singular */
         /* r^-7 and r^-13 by products (within a few ulp of pow, far cheaper) */
         const double ir2 = ir * ir, ir6 = ir2 * ir2 * ir2, ir7 = ir6 * ir, ir13 = ir6 * ir7;
         const double irc2 = irc * irc, irc6 = irc2 * irc2 * irc2, irc7 = irc6 * irc, irc13 = irc6 * irc7;

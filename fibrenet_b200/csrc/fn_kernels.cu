@@ -116,13 +116,14 @@ __device__ __forceinline__ void angle_arms(double bax, double bay, double baz, d
     const bool fast = fn_fast_range(ll);
     /* |dot| <= ll up to rounding: finite, and where it is too small for the
        quotient's residual the arc cosine does not see it */
-    double dotp = fast ? quotient(dot, ll, recip_from(ll, il_ba * il_bc)) : dot / ll;
+    double dotp = fast ? quotient(dot, ll, recip_near(ll, il_ba * il_bc)) : dot / ll;
     if (dotp < -1.0) dotp = -0.999999;
     if (dotp > 1.0) dotp = 0.999999;
     const double angle = acos_rounded(dotp);
     const double magnitude = -2.0 * (double)par.y * (angle - (double)par.x);
-    const double fa = fast ? quotient_any(magnitude, l_ba, il_ba) : magnitude / l_ba;
-    const double fc = fast ? quotient_any(magnitude, l_bc, il_bc) : magnitude / l_bc;
+    const bool fast_ends = fast && fn_quotient_range(magnitude);
+    const double fa = fast_ends ? quotient(magnitude, l_ba, il_ba) : magnitude / l_ba;
+    const double fc = fast_ends ? quotient(magnitude, l_bc, il_bc) : magnitude / l_bc;
     const double tx = bay * bcz - baz * bcy;
     const double ty = baz * bcx - bax * bcz;
     const double tz = bax * bcy - bay * bcx;
@@ -191,7 +192,7 @@ __device__ __forceinline__ int contact_law(const FnNet& N, const FnPair& law, do
             r = root_from(r2, y);
             if (!(r < P->c[2])) return 0;
             ir = recip_from(r, y);
-            const double ir2 = recip_from(r2, y * y);
+            const double ir2 = recip_near(r2, y * y);
             const double fr2 = quotient(P->lj_s2, r2, ir2);
             const double fr6 = fr2 * fr2 * fr2;
             fpr = quotient(P->lj_e48 * fr6 * (fr6 - 0.5), r2, ir2);

@@ -11,7 +11,8 @@
 
 using namespace fn;
 
-enum { OP_ROOT = 0, OP_INVERSE_ROOT = 1, OP_PRODUCT_INVERSE = 2, OP_SQUARE_INVERSE = 3, OP_QUOTIENT = 4, OP_QUOTIENT_ANY = 5 };
+enum { OP_ROOT = 0, OP_INVERSE_ROOT = 1, OP_PRODUCT_INVERSE = 2, OP_SQUARE_INVERSE = 3, OP_QUOTIENT = 4, OP_QUOTIENT_ANY = 5,
+       OP_SQUARE_QUOTIENT = 6 };
 
 static __global__ void k_rounded(int op, const double* a, const double* b, double* out, long long n) {
     const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
@@ -40,6 +41,10 @@ static __global__ void k_rounded(int op, const double* a, const double* b, doubl
         break;
     case OP_QUOTIENT_ANY: /* a / b for any a, b a finite root above 0 */
         r = quotient_any(a[i], b[i], 1.0 / b[i]);
+        break;
+    case OP_SQUARE_QUOTIENT: /* a / b from the seed of b's root, as a contact's quotients by its squared distance */
+        m = rsqrt_seeded(b[i]);
+        r = quotient(a[i], b[i], recip_near(b[i], m * m));
         break;
     }
     out[i] = r;

@@ -14,7 +14,8 @@ pytestmark = pytest.mark.gpu
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 HERE = os.path.join(ROOT, "tests", "rounded")
 HEADER = os.path.join(ROOT, "fibrenet_b200", "csrc", "fn_rounded.cuh")
-OP_ROOT, OP_INVERSE_ROOT, OP_PRODUCT_INVERSE, OP_SQUARE_INVERSE, OP_QUOTIENT, OP_QUOTIENT_ANY = range(6)
+OP_ROOT, OP_INVERSE_ROOT, OP_PRODUCT_INVERSE, OP_SQUARE_INVERSE, OP_QUOTIENT, OP_QUOTIENT_ANY, \
+    OP_SQUARE_QUOTIENT = range(7)
 
 # 2^106 - k = product of the primes, k = 1 .. 16
 FACTORS = {
@@ -174,31 +175,38 @@ def test_inverse_of_a_product(run):
     same_bits(run(OP_PRODUCT_INVERSE, a, b), 1.0 / product, a, b)
 
 
+def numerators(b, k):
+    """The mantissas a for which a/b lies next to the middle m of two doubles:
+    a 2^54 - b m = k or a 2^53 - b m = k, b and k odd (an even b keeps its
+    quotients twice as far from any middle)."""
+    for p in (53, 54) if b % 2 else ():
+        m = -k * pow(b, -1, 1 << p) % (1 << p)
+        m += (1 << 53) if m < 1 << 53 and p == 53 else 0
+        a = (b * m + k) >> p
+        if (1 << 53) <= m < (1 << 54) and (1 << 52) <= a < (1 << 53):
+            yield a
+
+
 def hard_quotients(n, seed):
-    """Pairs a, b whose quotient lies next to the middle m of two doubles:
-    a 2^54 - b m = k or a 2^53 - b m = k for small odd k."""
     rng = np.random.default_rng(seed)
     out = []
     while len(out) < n:
         b = int(rng.integers(1 << 52, 1 << 53)) | 1
-        k = int(rng.integers(-8, 8)) * 2 + 1
-        for p in (53, 54):
-            m = -k * pow(b, -1, 1 << p) % (1 << p)
-            m += (1 << 53) if m < 1 << 53 and p == 53 else 0
-            a = (b * m + k) >> p
-            if m & 1 and (1 << 53) <= m < (1 << 54) and (1 << 52) <= a < (1 << 53):
-                out.append((a, b))
+        out += [(a, b) for a in numerators(b, int(rng.integers(-8, 8)) * 2 + 1)]
+    for b in np.ldexp(hard_reciprocals(), 52).astype(np.int64):
+        out += [(a, int(b)) for k in range(-15, 16, 2) for a in numerators(int(b), k)]
     a, b = np.array(out, np.float64).T
     return np.ldexp(a, -52), np.ldexp(b, -52)
 
 
-def test_quotient(run):
+@pytest.mark.parametrize("op", [OP_QUOTIENT, OP_SQUARE_QUOTIENT])
+def test_quotient(run, op):
     ha, hb = hard_quotients(60_000, 7)
     rb = hard_reciprocals()
     rng = np.random.default_rng(8)
     a = np.concatenate([ha, -ha, 1.0 + rng.random(rb.size * 50), randoms(4_000_000, -200, 200, 9)])
     b = np.concatenate([hb, hb, np.repeat(rb, 50), randoms(4_000_000, -200, 200, 10)])
-    same_bits(run(OP_QUOTIENT, a, b), a / b, a, b)
+    same_bits(run(op, a, b), a / b, a, b)
 
 
 def test_quotient_of_any_numerator(run):

@@ -795,9 +795,9 @@ int build_bricks(fn_ctx* c) {
 
 /* Block size (and, for the staged chain kernel, contact items per thread and
    round) of the step kernel: tiles, per-tile tables and kernel attributes.
-   items_per_thread 0 selects the plain chain kernel; `wide` its form with
-   five warps per 28 beads, for contexts small enough. */
-int set_block(fn_ctx* c, int block, int items_per_thread, bool wide = false) {
+   items_per_thread 0 selects the plain chain kernel, or at the default block
+   size, for contexts small enough, its form with five warps per 28 beads. */
+int set_block(fn_ctx* c, int block, int items_per_thread) {
     if (c->chain && block > fn::kChainMaxBlock)
         return fail(c, FN_ERR_ARG, "block size " + std::to_string(block) + ": the chain step kernel takes at most " +
                                        std::to_string(fn::kChainMaxBlock) + " threads per block");
@@ -845,7 +845,7 @@ int set_block(fn_ctx* c, int block, int items_per_thread, bool wide = false) {
     CK(cudaStreamSynchronize(c->stream));
     c->ntiles = n;
     c->block = block;
-    c->wide = wide && c->chain && !c->staged && c->nb <= fn::kWideContext;
+    c->wide = c->chain && !c->staged && block == fn::kWideBlock && c->nb <= fn::kWideContext;
     return FN_OK;
 }
 
@@ -1564,7 +1564,7 @@ static int upload_host(fn_ctx* c, int n_networks, const fn_network_desc* nets) {
     int r = build_bricks(c);
     if (r) return r;
     r = set_block(c, c->cfg.block_size > 0 ? c->cfg.block_size : 128,
-                  c->cfg.chain_mode == 0 ? kDefaultItemsPerThread : 0, c->cfg.block_size == 0);
+                  c->cfg.chain_mode == 0 ? kDefaultItemsPerThread : 0);
     if (r) return r;
     r = verlet_setup(c);
     if (r) return r;
@@ -1845,8 +1845,7 @@ static int upload_device(fn_ctx* c, int n_networks, const fn_network_desc* nets)
     c->uploaded_on_device = true;
     r = build_bricks(c);
     if (r) return r;
-    r = set_block(c, c->cfg.block_size > 0 ? c->cfg.block_size : 128, c->cfg.chain_mode == 0 ? kDefaultItemsPerThread : 0,
-                  c->cfg.block_size == 0);
+    r = set_block(c, c->cfg.block_size > 0 ? c->cfg.block_size : 128, c->cfg.chain_mode == 0 ? kDefaultItemsPerThread : 0);
     if (r) return r;
     r = verlet_setup(c);
     if (r) return r;
@@ -2583,8 +2582,7 @@ FN_API int fn_autotune(fn_ctx* c, int steps_per_trial) {
     const long long steps0 = c->steps_done, rb0 = c->rebuilds_done;
     const bool timing0 = c->timing;
     c->timing = false;
-    std::vector<std::pair<int, int>> shapes; /* block, items per thread (-1: the wide form) */
-    if (c->chain && c->nb <= fn::kWideContext) shapes.emplace_back(128, -1);
+    std::vector<std::pair<int, int>> shapes; /* block, items per thread */
     for (int b : {64, 96, 128, 192, 256, 384, 512}) {
         if (c->chain && b > fn::kChainMaxBlock) continue;
         if (c->chain && c->cfg.chain_mode == 0)
@@ -2594,14 +2592,14 @@ FN_API int fn_autotune(fn_ctx* c, int steps_per_trial) {
     int dev = 0, optin = 0;
     CK(cudaGetDevice(&dev));
     CK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-    std::pair<int, int> best{c->block, c->wide ? -1 : c->staged ? c->chunk / c->block : 0};
+    std::pair<int, int> best{c->block, c->staged ? c->chunk / c->block : 0};
     float best_ms = 1e30f;
     cudaEvent_t e0, e1;
     CK(cudaEventCreate(&e0));
     CK(cudaEventCreate(&e1));
     for (const auto& sh : shapes) {
         if (sh.second > 0 && fn::step_staged_smem(sh.first, sh.first * sh.second) > (size_t)optin) continue;
-        if ((r = set_block(c, sh.first, std::max(sh.second, 0), sh.second < 0))) break;
+        if ((r = set_block(c, sh.first, sh.second))) break;
         for (int rep = 0; rep < 2 && !r; ++rep) { /* first run warms up */
             c->cur = cur0;
             for (auto& sn : snaps)
@@ -2622,7 +2620,7 @@ FN_API int fn_autotune(fn_ctx* c, int steps_per_trial) {
     /* then the list build (bead by bead, by bricks, by groups of lanes) at
        that shape */
     int best_build = c->list_build;
-    if (!r && (r = set_block(c, best.first, std::max(best.second, 0), best.second < 0)) == 0) {
+    if (!r && (r = set_block(c, best.first, best.second)) == 0) {
         float ms_build[3] = {1e30f, 1e30f, 1e30f};
         for (int mode = 0; mode < 3 && !r; ++mode) {
             c->list_build = mode;
@@ -2657,7 +2655,7 @@ FN_API int fn_autotune(fn_ctx* c, int steps_per_trial) {
     c->rebuilds_done = rb0;
     c->timing = timing0;
     if (r) return r;
-    return set_block(c, best.first, std::max(best.second, 0), best.second < 0);
+    return set_block(c, best.first, best.second);
     FN_CATCH(c)
 }
 

@@ -85,13 +85,15 @@ inline size_t step_tiled_smem(int max_sp, int max_an) {
            (size_t)max_sp + (size_t)max_an + 16;
 }
 
-/* Largest context (beads) whose default chain step is the wide form.  80 steps
+/* Largest context (beads) whose chain step at the default block size is the
+   wide form: block 128 names it there, its tiles are those of 128 threads.  80 steps
    with 10 rebuilds, wide against one thread per bead: 480 beads 475 / 675 us,
    10k 586 / 1010, dense 20k 892 / 1420, tensile 30k 1100 / 1376, 40k 940 /
    1106, tensile 60k 1470 / 1509, dense 100k 2422 / 1875: it needs about 44k
    beads' worth of blocks to fill the device twice, and then loses what it
-   gains.  A block size given by the caller is kept (no wide form). */
+   gains.  The other block sizes keep one thread per bead. */
 constexpr int kWideContext = 50000;
+constexpr int kWideBlock = 128;
 
 /* largest block the chain step kernel is built for (its launch bounds) */
 constexpr int kChainMaxBlock = 256;

@@ -443,7 +443,9 @@ class Simulation:
 
     def set_kernel_shape(self, block: int, items_per_thread: int = 0) -> None:
         """Step-kernel shape: block size and, for the staged chain kernel,
-        contact items per thread and round (0: no staging)."""
+        contact items per thread and round (0: no staging), as stats() reports
+        them.  Block 128 on the chain path steps contexts of at most 50,000
+        beads with five warps per 28 beads."""
         self._check(self.lib.fn_set_kernel_shape(self.h, int(block), int(items_per_thread)))
 
     LIST_BUILDS = ("beads", "bricks", "groups")

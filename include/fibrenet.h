@@ -115,13 +115,15 @@ typedef struct fn_config {
     int reorder;        /* 1: renumber beads in Morton order of their fibre */
     int use_graphs;     /* 1: replay steps as CUDA graphs */
     int block_size;     /* threads per block for the step kernel; 0 = default
-                           (128, and on the chain path contexts of at most
-                           50,000 beads step with five warps per 28 beads);
-                           at most 256 on the chain path */
+                           (128); at most 256 on the chain path.  There 128
+                           steps contexts of at most 50,000 beads with five
+                           warps per 28 beads, the other sizes, and 128 in
+                           larger contexts, with one thread per bead */
     int chain_mode;     /* 0 auto: per-bead bond records when the model is in
-                           chain form (fibres), the tile's data staged in
-                           shared memory before use; 1 chain form without
-                           staging; 2 never (incidence lists) */
+                           chain form (fibres), with fn_autotune and
+                           fn_set_kernel_shape free to stage the tile's data
+                           in shared memory first; 1 chain form, never staged;
+                           2 never (incidence lists) */
     double verlet_skin; /* 0: the reference's cadence (rebuild every
                            grid_update_freq steps, counter local to each
                            fn_step call, SimulationManager.cpp:152-173).
@@ -362,7 +364,8 @@ FN_API int fn_device_view(fn_ctx* ctx, int field, fn_view* out);
    items per thread and round, or no staging) from one snapshot of the state,
    restored after every trial, keeps the fastest, then keeps the fastest of
    the three list builds (fn_set_list_build) at that shape; the simulation
-   does not advance. */
+   does not advance.  fn_get_stats reports the choice; fn_set_kernel_shape and
+   fn_set_list_build with those numbers make it again. */
 FN_API int fn_autotune(fn_ctx* ctx, int steps_per_trial);
 
 /* How contact lists are built (ResetGrid .. BuildContactList,
@@ -376,8 +379,9 @@ FN_API int fn_set_list_build(fn_ctx* ctx, int mode);
 /* Sets the step kernel's shape: threads per block (a multiple of 32; 64 ..
    256 on the chain path, whose tiles hold block - 4 beads) and, for the
    staged chain kernel (chain_mode 0), contact items per thread and round
-   (1 .. 8; 0 runs the chain kernel without staging).  fn_autotune picks the
-   same parameters by timing. */
+   (1 .. 8; 0 runs the chain kernel without staging, at block 128 in contexts
+   of at most 50,000 beads with five warps per 28 beads).  fn_autotune picks
+   the same parameters by timing. */
 FN_API int fn_set_kernel_shape(fn_ctx* ctx, int block, int items_per_thread);
 
 /* Device-side snapshot of the dynamic state (positions, images, velocities,

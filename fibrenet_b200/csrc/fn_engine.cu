@@ -62,7 +62,10 @@ double list_r2(const NetHost& h, double cutoff_sq, double smax) {
    to every pair within the radius when the box is longer than the radius and
    two cells (a pair in neighbouring cells is at most two cells apart), and to
    every pair when moreover two cells are less than half of the shortest side
-   and the box longer than four cells. */
+   and the box longer than four cells.  On shorter boxes (three cells about as
+   wide as the radius) it takes the smaller of d and the box side less d along
+   each periodic axis instead (list_fold): no image is nearer, so what it
+   rejects is rejected, and every other pair is tested in FP64. */
 void set_list_radii(FnNet& N, const NetHost& h, double smax, double rmin, double smin) {
     N.list_r2_max = list_r2(h, N.list_cut_sq, smax);
     const double err = std::max({N.box[0], N.box[1], N.box[2]}) * std::ldexp(1.0, -21);
@@ -74,14 +77,17 @@ void set_list_radii(FnNet& N, const NetHost& h, double smax, double rmin, double
     if (h.kinds & 1u << FN_PAIR_HS) in = std::min(in, hs);
     if (h.kinds & 1u << FN_PAIR_HSR) in = std::min(in, std::max(cut, hs));
     in -= err;
-    bool out_ok = out < 1e15, in_ok = in > 0.0 && in < 1e15 && !(h.kinds & 1u);
+    const bool out_ok = out < 1e15;
+    bool in_ok = in > 0.0 && in < 1e15 && !(h.kinds & 1u);
+    N.list_fold = 0;
     for (int a = 0; a < 3; ++a) {
         if (!(N.list_mi >> a & 1)) continue;
-        out_ok = out_ok && N.box[a] - 2.0 * N.step[a] > 1.001 * out;
+        if (!(N.box[a] - 2.0 * N.step[a] > 1.001 * out)) N.list_fold = 1;
         in_ok = in_ok && 2.001 * N.step[a] < 0.5 * shortest && N.box[a] > 4.001 * N.step[a];
     }
-    N.list_out_r2 = out_ok ? std::nextafter((float)(out * out * (1.0 + 1e-6)), std::numeric_limits<float>::infinity()) : -1.0f;
-    N.list_in_r2 = out_ok && in_ok ? std::nextafter((float)(in * in * (1.0 - 1e-6)), 0.0f) : -1.0f;
+    const float all = std::numeric_limits<float>::infinity();
+    N.list_out_r2 = out_ok ? std::nextafter((float)(out * out * (1.0 + 1e-6)), all) : all;
+    N.list_in_r2 = out_ok && in_ok && !N.list_fold ? std::nextafter((float)(in * in * (1.0 - 1e-6)), 0.0f) : -1.0f;
 }
 
 /* the skin radius the upload gives a bead */

@@ -1691,12 +1691,15 @@ __device__ __forceinline__ bool list_pair(const RebuildArgs& R, const FnNet& N, 
 }
 
 /* The second test of a near candidate (its index, the sign set when the first
-   test left its distance open): the exclusion of bonded neighbours, and where
-   the distance is open the test in FP64. */
+   test left its distance open): the exclusion of bonded neighbours, where the
+   distance is open the test in FP64, and where its row is long enough to hold
+   an overfull cell (crowded), that its cell has kept it. */
 template <bool UNIFORM>
-__device__ __forceinline__ bool list_second(const RebuildArgs& R, const FnNet& N, int i, int4 bi, int w, int& j) {
+__device__ __forceinline__ bool list_second(const RebuildArgs& R, const FnNet& N, int i, int4 bi, int w, bool crowded,
+                                            int& j) {
     j = w & 0x7fffffff;
     const int4 bj = R.binfo[j];
+    if (crowded && R.cell_of[j] < 0) return false;
     if (bi.x == bj.x && abs(bi.y - bj.y) <= 1) return false;
     return w >= 0 || list_pair<UNIFORM>(R, N, R.pos[i], bi, R.pos[j], bj);
 }
@@ -1744,6 +1747,18 @@ __device__ __forceinline__ void cell_coords(const FnNet& N, int c, int& cx, int&
 
 __device__ __forceinline__ void list_one_bead(const RebuildArgs& R, const FnNet& N, int i, int c);
 
+/* The longest run of three cells that the builds below take as one run of the
+   sorted array: at twice the beads that three full cells keep, testing the
+   dropped ones costs about as much as it saves to test in FP32. */
+__device__ __forceinline__ int longest_run(int cell_cap) { return 6 * min(cell_cap, 1 << 28); }
+
+/* Per axis the smaller of |d| and its distance from the box side (`side`,
+   infinite where the axis is not periodic): no image of the pair is nearer. */
+__device__ __forceinline__ float fold_axis(float d, float side) { return fminf(fabsf(d), fabsf(side - fabsf(d))); }
+__device__ __forceinline__ float fold_side(const FnNet& N, int a) {
+    return N.periodic >> a & 1 ? (float)N.box[a] : __int_as_float(0x7f800000);
+}
+
 /* Full per-bead lists over the 27-cell neighbourhood (dz, dy, dx ascending,
    beads ascending within a cell): the symmetric closure of the reference's
    half-shell pair set, in a fixed order.  G lanes of a warp work on one bead;
@@ -1758,8 +1773,11 @@ __device__ __forceinline__ void list_one_bead(const RebuildArgs& R, const FnNet&
      3. Second test: the near ones, G at a time, in FP64 with the pair law's
         radius and the exclusion of bonded neighbours; the accepted ones are
         written in order by a ballot over the group.
-   A bead whose rows may hold an overfull cell, and boxes too small for the
-   first test, go candidate by candidate in FP64 (list_one_bead).
+   A row with more beads than one cell may keep can hold an overfull cell; its
+   dropped beads, the last of their cell, fail the second test (whole rebuild,
+   100k beads at 22 per cell: 377 us, 788 when such rows took the FP64 test
+   candidate by candidate).  Beads next to a cell far over its capacity
+   (longest_run) are listed cell by cell, the kept beads G at a time, in FP64.
    A bead's loads are then a handful of dependent rounds instead of one per
    candidate, which is what small networks wait for. */
 /* A row's candidates: number k < end is entry (k < split ? a : b) + k; shift says
@@ -1793,7 +1811,8 @@ __global__ void __launch_bounds__(128, 10) k_lists_group(const __grid_constant__
     }
     const FnNet& N = UNIFORM ? R.net0 : R.nets[i >= 0 ? net_of_bead(R.nets, R.n_nets, i) : 0];
     const float r2 = N.list_out_r2;
-    bool plain = !(r2 >= 0.0f); /* no first test */
+    const bool fold = N.list_fold;
+    int widest = 0; /* beads of the fullest run */
     ListRow* rows = s_row + 9 * grp;
     unsigned char* shifts = s_shift + 9 * grp;
     int* near = s_near + kListNear * grp;
@@ -1837,7 +1856,7 @@ __global__ void __launch_bounds__(128, 10) k_lists_group(const __grid_constant__
                         nb = row[1] - b0;
                         shift |= 4;
                     }
-                    if (na > R.cell_cap || nb > R.cell_cap) plain = true;
+                    widest = max(widest, max(na, nb));
                 }
             }
             /* number the candidates: inclusive scan over the group's lanes */
@@ -1858,15 +1877,25 @@ __global__ void __launch_bounds__(128, 10) k_lists_group(const __grid_constant__
     }
     const unsigned gmask = G == 32 ? full : (((1u << G) - 1u) << (lane & ~(G - 1)));
     const unsigned below = (1u << lane) - 1u;
-    plain = (__ballot_sync(full, plain) & gmask) != 0;
-    moved = __any_sync(full, moved);
+    const bool plain = (__ballot_sync(full, widest > longest_run(R.cell_cap)) & gmask) != 0;
+    const bool crowded = __any_sync(full, widest > R.cell_cap);
+    moved = __any_sync(full, moved || fold);
     if (plain || i < 0) total = 0;
     __syncwarp();
     int4 bi = make_int4(0, 0, 0, 0);
-    if (total > 0) bi = R.binfo[i];
+    if (total > 0 || plain) bi = R.binfo[i];
     const float in_r2 = N.list_in_r2;
     int* __restrict__ out = R.list + (i >= 0 ? i : 0);
     int n = 0, m = 0;
+    /* writes the accepted candidates of the group's lanes, in order */
+    auto add = [&](bool acc, int j) {
+        const unsigned mine = __ballot_sync(full, acc) & gmask;
+        if (acc) {
+            const int at = n + __popc(mine & below);
+            if (at < R.list_cap) out[(size_t)at * R.list_stride] = j;
+        }
+        n += __popc(mine);
+    };
     /* second test of the m near candidates */
     auto flush = [&]() {
         __syncwarp();
@@ -1875,13 +1904,8 @@ __global__ void __launch_bounds__(128, 10) k_lists_group(const __grid_constant__
             const int k = k0 + gl;
             bool acc = false;
             int j = -1;
-            if (k < m) acc = list_second<UNIFORM>(R, N, i, bi, near[k], j);
-            const unsigned mine = __ballot_sync(full, acc) & gmask;
-            if (acc) {
-                const int at = n + __popc(mine & below);
-                if (at < R.list_cap) out[(size_t)at * R.list_stride] = j;
-            }
-            n += __popc(mine);
+            if (k < m) acc = list_second<UNIFORM>(R, N, i, bi, near[k], crowded, j);
+            add(acc, j);
         }
         m = 0;
         __syncwarp();
@@ -1899,14 +1923,20 @@ __global__ void __launch_bounds__(128, 10) k_lists_group(const __grid_constant__
             j = __float_as_int(e.w);
             float dx = o.x - e.x, dy = o.y - e.y, dz = o.z - e.z;
             if (moved) {
-                const int sh = shifts[r], sx = k < u.split ? sh : sh >> 2;
-                const float bx = (float)N.box[0], by = (float)N.box[1], bz = (float)N.box[2];
-                dx += sx & 1 ? -bx : sx & 2 ? bx : 0.0f;
-                dy += sh & 16 ? -by : sh & 32 ? by : 0.0f;
-                dz += sh & 64 ? -bz : sh & 128 ? bz : 0.0f;
+                if (fold) {
+                    dx = fold_axis(dx, fold_side(N, 0));
+                    dy = fold_axis(dy, fold_side(N, 1));
+                    dz = fold_axis(dz, fold_side(N, 2));
+                } else {
+                    const int sh = shifts[r], sx = k < u.split ? sh : sh >> 2;
+                    const float bx = (float)N.box[0], by = (float)N.box[1], bz = (float)N.box[2];
+                    dx += sx & 1 ? -bx : sx & 2 ? bx : 0.0f;
+                    dy += sh & 16 ? -by : sh & 32 ? by : 0.0f;
+                    dz += sh & 64 ? -bz : sh & 128 ? bz : 0.0f;
+                }
             }
             const float d2 = __fmaf_rn(dx, dx, __fmaf_rn(dy, dy, dz * dz));
-            hit = d2 <= r2 && j != i;
+            hit = !(d2 > r2) && j != i;
             if (!(d2 <= in_r2)) j |= (int)0x80000000;
         }
         const unsigned mine = __ballot_sync(full, hit) & gmask;
@@ -1915,14 +1945,49 @@ __global__ void __launch_bounds__(128, 10) k_lists_group(const __grid_constant__
         if (__any_sync(full, m > kListNear - G)) flush();
     }
     flush();
-    if (gl == 0 && i >= 0) {
-        if (plain) {
-            list_one_bead(R, N, i, c);
-        } else {
-            if (n > R.list_cap)
-                atomicAdd(R.counters + FN_CNT_LIST_OVERFLOW, (unsigned long long)(n - R.list_cap));
-            R.list_count[i] = n;
+    if (__any_sync(full, plain)) {
+        double4 pi = make_double4(0.0, 0.0, 0.0, 0.0);
+        if (plain) pi = R.pos[i];
+        int cx, cy, cz;
+        cell_coords(N, c, cx, cy, cz);
+        for (int d = 0; d < 27; ++d) {
+            int z = cz + d / 9 - 1, y = cy + d / 3 % 3 - 1, x = cx + d % 3 - 1;
+            bool ok = plain;
+            if (z < 0 || z >= N.nz) {
+                ok = ok && (N.periodic & 4);
+                z = z < 0 ? N.nz - 1 : 0;
+            }
+            if (y < 0 || y >= N.ny) {
+                ok = ok && (N.periodic & 2);
+                y = y < 0 ? N.ny - 1 : 0;
+            }
+            if (x < 0 || x >= N.nx) {
+                ok = ok && (N.periodic & 1);
+                x = x < 0 ? N.nx - 1 : 0;
+            }
+            int s = 0, kept = 0;
+            if (ok) {
+                const int* at = R.cell_start + (N.cell_base + x + y * N.nx + z * N.nxy);
+                s = at[0];
+                kept = min(at[1] - s, R.cell_cap);
+            }
+            const int rounds = __reduce_max_sync(full, kept);
+            for (int k0 = 0; k0 < rounds; k0 += G) {
+                const int k = k0 + gl;
+                bool acc = false;
+                int j = -1;
+                if (k < kept) {
+                    j = R.cell_beads[s + k];
+                    acc = list_pair<UNIFORM>(R, N, pi, bi, R.pos[j], R.binfo[j]);
+                }
+                add(acc, j);
+            }
         }
+    }
+    if (gl == 0 && i >= 0) {
+        if (n > R.list_cap)
+            atomicAdd(R.counters + FN_CNT_LIST_OVERFLOW, (unsigned long long)(n - R.list_cap));
+        R.list_count[i] = n;
     }
 }
 
@@ -1941,7 +2006,7 @@ __global__ void __launch_bounds__(128, 8) k_lists(const __grid_constant__ Rebuil
     await_previous();
     FN_GATED(R.gate);
     __shared__ int s_first[9 * 128];
-    __shared__ unsigned char s_len[9 * 128];
+    __shared__ unsigned short s_len[9 * 128];
     __shared__ int s_near[kListKeep * 128];
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= R.cell_start[ncells]) return; /* beads placed in the grid */
@@ -1952,11 +2017,11 @@ __global__ void __launch_bounds__(128, 8) k_lists(const __grid_constant__ Rebuil
     const FnNet& N = UNIFORM ? R.net0 : R.nets[net_of_bead(R.nets, R.n_nets, i)];
     const float out_r2 = N.list_out_r2, in_r2 = N.list_in_r2;
     int* first = s_first + threadIdx.x;
-    unsigned char* len = s_len + threadIdx.x;
+    unsigned short* len = s_len + threadIdx.x;
     int* near = s_near + threadIdx.x;
     int cx, cy, cz;
     cell_coords(N, c, cx, cy, cz);
-    const int cap = min(R.cell_cap, 255);
+    const int longest = min(longest_run(R.cell_cap), 65535); /* s_len */
     /* the nine rows (dz, dy ascending): the row's cells in place are one run
        of the sorted arrays; all cell starts are loaded together */
     const int xa = max(cx - 1, 0), xb = min(cx + 2, N.nx);
@@ -1964,7 +2029,7 @@ __global__ void __launch_bounds__(128, 8) k_lists(const __grid_constant__ Rebuil
     const int zhi = cz + 1 < N.nz ? N.nxy : N.periodic & 4 ? -cz * N.nxy : INT_MIN;
     const int ylo = cy > 0 ? -N.nx : N.periodic & 2 ? (N.ny - 1) * N.nx : INT_MIN;
     const int yhi = cy + 1 < N.ny ? N.nx : N.periodic & 2 ? -cy * N.nx : INT_MIN;
-    bool plain = !(out_r2 >= 0.0f);
+    int widest = 0;
     const int* own = R.cell_start + (c - cx);
     {
         int s0[9], s1[9];
@@ -1978,15 +2043,17 @@ __global__ void __launch_bounds__(128, 8) k_lists(const __grid_constant__ Rebuil
         }
 #pragma unroll
         for (int k = 0; k < 9; ++k) {
-            plain = plain || s1[k] - s0[k] > cap;
+            widest = max(widest, s1[k] - s0[k]);
             first[128 * k] = s0[k];
-            len[128 * k] = (unsigned char)(s1[k] - s0[k]);
+            len[128 * k] = (unsigned short)(s1[k] - s0[k]);
         }
     }
     /* beyond a periodic side in x, one more cell of each row, before or after
        the others */
     const bool wl = cx == 0 && (N.periodic & 1), wr = cx + 1 == N.nx && (N.periodic & 1);
     const bool moved = wl || wr || (cz == 0 || cz + 1 == N.nz) || (cy == 0 || cy + 1 == N.ny);
+    const bool fold = N.list_fold; /* then the bead stays where it is */
+    const float bx = fold ? 0.0f : (float)N.box[0], by = fold ? 0.0f : (float)N.box[1], bz = fold ? 0.0f : (float)N.box[2];
     const int4 bi = R.binfo[i];
     int* __restrict__ out = R.list + i;
     int n = 0, m = 0;
@@ -1994,29 +2061,34 @@ __global__ void __launch_bounds__(128, 8) k_lists(const __grid_constant__ Rebuil
     auto flush = [&]() {
         for (int k = 0; k < m; ++k) {
             int j;
-            if (list_second<UNIFORM>(R, N, i, bi, near[128 * k], j)) { /* i itself is excluded, as a bonded neighbour */
+            if (list_second<UNIFORM>(R, N, i, bi, near[128 * k], widest > R.cell_cap, j)) { /* i itself is excluded, as a bonded neighbour */
                 if (n < R.list_cap) out[(size_t)n * R.list_stride] = j;
                 ++n;
             }
         }
         m = 0;
     };
-    for (int k = 0; k < 9 && !plain; ++k) {
+    /* first test of a candidate (dx, dy, dz) away */
+    auto keep = [&](float4 v, float dx, float dy, float dz) {
+        const float d2 = __fmaf_rn(dx, dx, __fmaf_rn(dy, dy, dz * dz));
+        if (!(d2 > out_r2)) near[128 * m++] = __float_as_int(v.w) | (d2 <= in_r2 ? 0 : (int)0x80000000);
+    };
+    for (int k = 0; k < 9 && widest <= longest; ++k) {
         float ox = o.x, oy = o.y, oz = o.z;
         int q = first[128 * k], left = len[128 * k];
         int q2 = 0, left2 = 0;
         if (moved) {
             /* cells below the grid lie at the far side: the bead moves up */
             const int dz = k < 3 ? zlo : k < 6 ? 0 : zhi, dy = k % 3 == 0 ? ylo : k % 3 == 1 ? 0 : yhi;
-            if (k < 3 && cz == 0) oz += (float)N.box[2];
-            if (k >= 6 && cz + 1 == N.nz) oz -= (float)N.box[2];
-            if (k % 3 == 0 && cy == 0) oy += (float)N.box[1];
-            if (k % 3 == 2 && cy + 1 == N.ny) oy -= (float)N.box[1];
+            if (k < 3 && cz == 0) oz += bz;
+            if (k >= 6 && cz + 1 == N.nz) oz -= bz;
+            if (k % 3 == 0 && cy == 0) oy += by;
+            if (k % 3 == 2 && cy + 1 == N.ny) oy -= by;
             if ((wl || wr) && dz != INT_MIN && dy != INT_MIN) {
                 const int* w = own + dz + dy + (wl ? N.nx - 1 : 0);
                 q2 = w[0];
                 left2 = w[1] - q2;
-                if (left2 > cap) plain = true;
+                widest = max(widest, left2);
                 if (wl) { /* first */
                     int v = q;
                     q = q2;
@@ -2024,7 +2096,7 @@ __global__ void __launch_bounds__(128, 8) k_lists(const __grid_constant__ Rebuil
                     v = left;
                     left = left2;
                     left2 = v;
-                    ox += (float)N.box[0];
+                    ox += bx;
                 }
             }
         }
@@ -2033,22 +2105,29 @@ __global__ void __launch_bounds__(128, 8) k_lists(const __grid_constant__ Rebuil
                 if (m + left > kListKeep) flush();
                 const int stop = q + min(left, kListKeep);
                 left -= stop - q;
+                if (fold) {
+                    const float fx = fold_side(N, 0), fy = fold_side(N, 1), fz = fold_side(N, 2);
+#pragma unroll 2
+                    for (; q < stop; ++q) {
+                        const float4 v = R.cell_pos[q];
+                        keep(v, fold_axis(ox - v.x, fx), fold_axis(oy - v.y, fy), fold_axis(oz - v.z, fz));
+                    }
+                    continue;
+                }
 #pragma unroll 2
                 for (; q < stop; ++q) {
                     const float4 v = R.cell_pos[q];
-                    const float dx = ox - v.x, dy = oy - v.y, dz = oz - v.z;
-                    const float d2 = __fmaf_rn(dx, dx, __fmaf_rn(dy, dy, dz * dz));
-                    if (d2 <= out_r2) near[128 * m++] = __float_as_int(v.w) | (d2 <= in_r2 ? 0 : (int)0x80000000);
+                    keep(v, ox - v.x, oy - v.y, oz - v.z);
                 }
             }
             if (left2 == 0) break;
             q = q2;
             left = left2;
             left2 = 0;
-            ox = wl ? o.x : o.x - (float)N.box[0];
+            ox = wl ? o.x : o.x - bx;
         }
     }
-    if (plain) {
+    if (widest > longest) {
         list_one_bead(R, N, i, c); /* candidate by candidate in FP64 */
         return;
     }

@@ -34,12 +34,14 @@ struct FnNet {
     int pair_base;   /* first entry of this network in the pair table */
     int bead_begin, bead_end;
     float list_out_r2;  /* FP32 positions further apart than this (squared)
-                           belong to no listed pair; negative: no such test */
+                           belong to no listed pair; infinite: no such test */
     float list_in_r2;   /* and no further than this: within the listing radius
                            of every pair law; negative: no such test */
     unsigned div_nx, div_nxy;     /* c / nx = umulhi(c, div_nx) >> shift_nx for */
     int shift_nx, shift_nxy;      /* every cell index c >= 0, likewise nxy */
-    int pad_;
+    int list_fold;   /* FP32 separations are folded into half the box: some
+                        periodic axis is too short to tell the images apart by
+                        the cells */
     double list_r2_max; /* no pair further apart than this (squared) is listed */
     double list_cut_sq; /* listing radius of cut-off pair kinds (squared): the
                            cut-off, plus the Verlet skin in displacement mode */

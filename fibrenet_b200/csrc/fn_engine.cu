@@ -9,6 +9,8 @@
  */
 #include <cuda_runtime.h>
 #include <sched.h>
+#include <sys/mman.h>
+#include <unistd.h>
 
 #include <algorithm>
 #include <atomic>
@@ -1975,13 +1977,32 @@ FN_API int fn_device_view(fn_ctx* c, int field, fn_view* out) {
     FN_CATCH(c)
 }
 
+/* Whether some page of a mapped range is still to be faulted in.  False where
+   the range is not mapped or the kernel does not tell. */
+static bool pages_missing(const void* buffer, size_t bytes) {
+    const size_t page = (size_t)sysconf(_SC_PAGESIZE);
+    unsigned char there[4096];
+    const uintptr_t end = (uintptr_t)buffer + bytes;
+    for (uintptr_t at = (uintptr_t)buffer / page * page; at < end;) {
+        const size_t n = std::min<size_t>(sizeof there, (end - at + page - 1) / page);
+        if (mincore((void*)at, n * page, there) != 0) return false;
+        for (size_t k = 0; k < n; ++k)
+            if (!(there[k] & 1)) return true;
+        at += n * page;
+    }
+    return false;
+}
+
 /* Touches every page of a buffer that a copy is about to fill, on host threads:
    the pages of a large fresh allocation are mapped one fault after the other
-   otherwise, inside the copy (76 MB: 17.7 ms, 4.4 with the pages present),
+   otherwise, inside the copy (76 MB: 17.2 ms, 4.6 with the pages present),
    while here the device is still busy with what the copy waits for.  Bytes
    keep their values.  Only the caller's pageable memory: pinned pages are
-   there, and any other address is the copy's to take or refuse. */
+   there, and any other address is the copy's to take or refuse.  Only where a
+   page is missing: touching present ones costs 0.3 ms of a 0.9 ms copy of
+   17 MB. */
 static void touch_pages(void* buffer, size_t bytes) {
+    if (!pages_missing(buffer, bytes)) return;
     cudaPointerAttributes at{};
     if (cudaPointerGetAttributes(&at, buffer) != cudaSuccess) {
         (void)cudaGetLastError();

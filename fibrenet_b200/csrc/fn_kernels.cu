@@ -17,8 +17,9 @@
  * with deterministic order.
  *
  * All force arithmetic is FP64 with the reference's operation order; the
- * library is built with -fmad=false so nothing is contracted into FMAs, which
- * keeps results bit-identical to the host mirror checker.
+ * library is built with -fmad=false so nothing is contracted into FMAs, and
+ * the roots, reciprocals and quotients of fn_rounded.cuh round as the operators
+ * do, which keeps results bit-identical to the host mirror checker.
  */
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -332,8 +333,6 @@ __device__ __forceinline__ void base_force(const StepArgs& A, const FnNet& N, in
    that the chain kernel's forces-only form evaluates. */
 enum { FN_STEP_SPRINGS = 1, FN_STEP_ANGLES = 2, FN_STEP_CONTACTS = 4, FN_STEP_DRIFT = 8, FN_STEP_STORE_V = 16 };
 
-/* AdvanceVelocity and the next AdvancePosition for bead i with its complete
-   force (Fx, Fy, Fz), then the stores. */
 /* What the kick reads of bead i: its image position, force and velocity_old. */
 struct KickState {
     double4 im;
@@ -344,6 +343,8 @@ __device__ __forceinline__ KickState kick_state(const StepArgs& A, int i) {
     return KickState{A.img_in[i], A.force[i], A.vold[i]};
 }
 
+/* AdvanceVelocity and the next AdvancePosition for bead i with its complete
+   force (Fx, Fy, Fz), then the stores. */
 template <bool DAMP>
 __device__ __forceinline__ void kick_drift(const StepArgs& A, const FnNet& N, int i, double4 p, double Fx, double Fy,
                                            double Fz, KickState k, bool do_drift, bool store_v) {
@@ -1505,7 +1506,6 @@ __global__ void k_reset_energy(float4* force, float4* vel, float4* vold, int n) 
 /* ------------------------------------------------------------------------ */
 /* Contact-list rebuild                                                      */
 
-/* FillGrid's cell computation (kernel.cl:492-501) + per-cell counting. */
 /* Displacement-triggered mode: every rebuild kernel returns at once unless
    the device gate says a rebuild is due (a null gate always rebuilds). */
 #define FN_GATED(g)                   \
@@ -1521,6 +1521,7 @@ __global__ void k_fill_int(int* p, long long n, int v, const int* gate) {
         p[i] = v;
 }
 
+/* FillGrid's cell computation (kernel.cl:492-501) + per-cell counting. */
 __global__ void k_cells(const RebuildArgs R) {
     await_previous();
     let_next_start();
@@ -1759,6 +1760,16 @@ __device__ __forceinline__ float fold_side(const FnNet& N, int a) {
     return N.periodic >> a & 1 ? (float)N.box[a] : __int_as_float(0x7f800000);
 }
 
+/* A row's candidates: number k < end is entry (k < split ? a : b) + k; shift says
+   how the bead moves for them, two bits per axis (1 down by the box, 2 up),
+   bits 0-1 for the first part in x, 2-3 for the second, 4-5 y, 6-7 z. */
+struct ListRow {
+    int a, b, split, end;
+};
+
+/* The near candidates a group keeps between the tests. */
+constexpr int kListNear = 32;
+
 /* Full per-bead lists over the 27-cell neighbourhood (dz, dy, dx ascending,
    beads ascending within a cell): the symmetric closure of the reference's
    half-shell pair set, in a fixed order.  G lanes of a warp work on one bead;
@@ -1780,16 +1791,6 @@ __device__ __forceinline__ float fold_side(const FnNet& N, int a) {
    (longest_run) are listed cell by cell, the kept beads G at a time, in FP64.
    A bead's loads are then a handful of dependent rounds instead of one per
    candidate, which is what small networks wait for. */
-/* A row's candidates: number k < end is entry (k < split ? a : b) + k; shift says
-   how the bead moves for them, two bits per axis (1 down by the box, 2 up),
-   bits 0-1 for the first part in x, 2-3 for the second, 4-5 y, 6-7 z. */
-struct ListRow {
-    int a, b, split, end;
-};
-
-/* The near candidates a group keeps between the tests. */
-constexpr int kListNear = 32;
-
 template <int G, bool UNIFORM>
 __global__ void __launch_bounds__(128, 10) k_lists_group(const __grid_constant__ RebuildArgs R, long long ncells) {
     await_previous();
@@ -2488,9 +2489,7 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan_partials(const int* in, l
 }
 
 /* One block scans the block sums in chunks, carrying the running total. */
-__global__ void __launch_bounds__(SCAN_THREADS) k_scan_sums(int* block_sums, int nblocks,
-                                                             int* grand_total, const int* gate) {
-    FN_GATED(gate);
+__global__ void __launch_bounds__(SCAN_THREADS) k_scan_sums(int* block_sums, int nblocks, int* grand_total) {
     __shared__ int ws[33];
     int carry = 0;
     for (int base = 0; base < nblocks; base += SCAN_THREADS) {
@@ -2504,13 +2503,10 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan_sums(int* block_sums, int
     if (threadIdx.x == 0) *grand_total = carry;
 }
 
-/* Exclusive scan, last pass: each block's offset added, written to out;
-   zero (if given) is cleared alongside, sparing a launch. */
+/* Exclusive scan, last pass: each block's offset added, written to out. */
 template <int SCAN_ITEMS>
 __global__ void __launch_bounds__(SCAN_THREADS) k_scan_apply(const int* in, long long n,
-                                                              const int* block_sums, int* out,
-                                                              const int* gate, int* zero) {
-    FN_GATED(gate);
+                                                              const int* block_sums, int* out) {
     __shared__ int ws[33];
     const long long base = (long long)blockIdx.x * (SCAN_THREADS * SCAN_ITEMS) + (long long)threadIdx.x * SCAN_ITEMS;
     int v[SCAN_ITEMS];
@@ -2520,7 +2516,7 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan_apply(const int* in, long
     for (int k = 0; k < SCAN_ITEMS; ++k) s += v[k];
     int total;
     const int ex = block_exclusive_scan(s, ws, total) + block_sums[blockIdx.x];
-    scan_finish<SCAN_ITEMS>(out, zero, base, n, v, ex);
+    scan_finish<SCAN_ITEMS>(out, nullptr, base, n, v, ex);
 }
 
 /* Exclusive scan, last pass, without a pass of its own over the block sums:
@@ -2818,8 +2814,8 @@ template <int ITEMS>
 static void launch_scan(const int* in, long long n, int* out, int* block_sums, cudaStream_t s) {
     const unsigned nblk = (unsigned)scan_block_count(n);
     k_scan_partials<ITEMS><<<nblk, SCAN_THREADS, 0, s>>>(in, n, block_sums, nullptr);
-    k_scan_sums<<<1, SCAN_THREADS, 0, s>>>(block_sums, (int)nblk, out + n, nullptr);
-    k_scan_apply<ITEMS><<<nblk, SCAN_THREADS, 0, s>>>(in, n, block_sums, out, nullptr, nullptr);
+    k_scan_sums<<<1, SCAN_THREADS, 0, s>>>(block_sums, (int)nblk, out + n);
+    k_scan_apply<ITEMS><<<nblk, SCAN_THREADS, 0, s>>>(in, n, block_sums, out);
 }
 
 cudaError_t launch_exclusive_scan(const int* in, long long n, int* out, int* block_sums, cudaStream_t s) {

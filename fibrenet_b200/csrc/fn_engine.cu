@@ -939,6 +939,7 @@ fn::RebuildArgs rebuild_args(fn_ctx* c) {
     R.cell_beads = c->cell_beads.p;
     R.cell_raw = c->cell_raw.p;
     R.cell_pos = c->cell_pos.p;
+    for (const FnNet& N : c->nets_h) R.fold |= N.list_fold;
     R.uniform = c->uniform;
     if (c->uniform != fn::FN_CONST_NONE) {
         R.net0 = c->nets_h[0];

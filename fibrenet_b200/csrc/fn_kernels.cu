@@ -2002,7 +2002,7 @@ constexpr int kListKeep = 24;
    where it cannot decide, took the rebuild of the 1M-bead tensile network
    from 313 to 211 us and that of the 4M-bead mat from 1,340 to 943 us (202
    and 904 since its launches are chained and its scan reads wider). */
-template <bool UNIFORM>
+template <bool UNIFORM, bool FOLD>
 __global__ void __launch_bounds__(128, 8) k_lists(const __grid_constant__ RebuildArgs R, long long ncells) {
     await_previous();
     FN_GATED(R.gate);
@@ -2053,21 +2053,26 @@ __global__ void __launch_bounds__(128, 8) k_lists(const __grid_constant__ Rebuil
        the others */
     const bool wl = cx == 0 && (N.periodic & 1), wr = cx + 1 == N.nx && (N.periodic & 1);
     const bool moved = wl || wr || (cz == 0 || cz + 1 == N.nz) || (cy == 0 || cy + 1 == N.ny);
-    const bool fold = N.list_fold; /* then the bead stays where it is */
-    const float bx = fold ? 0.0f : (float)N.box[0], by = fold ? 0.0f : (float)N.box[1], bz = fold ? 0.0f : (float)N.box[2];
+    const bool fold = FOLD && N.list_fold; /* then the bead stays where it is */
     const int4 bi = R.binfo[i];
     int* __restrict__ out = R.list + i;
     int n = 0, m = 0;
     /* second test of the near candidates */
-    auto flush = [&]() {
+    auto test = [&](bool crowded) {
         for (int k = 0; k < m; ++k) {
             int j;
-            if (list_second<UNIFORM>(R, N, i, bi, near[128 * k], widest > R.cell_cap, j)) { /* i itself is excluded, as a bonded neighbour */
+            if (list_second<UNIFORM>(R, N, i, bi, near[128 * k], crowded, j)) { /* i itself is excluded, as a bonded neighbour */
                 if (n < R.list_cap) out[(size_t)n * R.list_stride] = j;
                 ++n;
             }
         }
         m = 0;
+    };
+    auto flush = [&]() {
+        if (widest > R.cell_cap)
+            test(true);
+        else
+            test(false);
     };
     /* first test of a candidate (dx, dy, dz) away */
     auto keep = [&](float4 v, float dx, float dy, float dz) {
@@ -2081,10 +2086,12 @@ __global__ void __launch_bounds__(128, 8) k_lists(const __grid_constant__ Rebuil
         if (moved) {
             /* cells below the grid lie at the far side: the bead moves up */
             const int dz = k < 3 ? zlo : k < 6 ? 0 : zhi, dy = k % 3 == 0 ? ylo : k % 3 == 1 ? 0 : yhi;
-            if (k < 3 && cz == 0) oz += bz;
-            if (k >= 6 && cz + 1 == N.nz) oz -= bz;
-            if (k % 3 == 0 && cy == 0) oy += by;
-            if (k % 3 == 2 && cy + 1 == N.ny) oy -= by;
+            if (!fold) {
+                if (k < 3 && cz == 0) oz += (float)N.box[2];
+                if (k >= 6 && cz + 1 == N.nz) oz -= (float)N.box[2];
+                if (k % 3 == 0 && cy == 0) oy += (float)N.box[1];
+                if (k % 3 == 2 && cy + 1 == N.ny) oy -= (float)N.box[1];
+            }
             if ((wl || wr) && dz != INT_MIN && dy != INT_MIN) {
                 const int* w = own + dz + dy + (wl ? N.nx - 1 : 0);
                 q2 = w[0];
@@ -2097,7 +2104,7 @@ __global__ void __launch_bounds__(128, 8) k_lists(const __grid_constant__ Rebuil
                     v = left;
                     left = left2;
                     left2 = v;
-                    ox += bx;
+                    if (!fold) ox += (float)N.box[0];
                 }
             }
         }
@@ -2125,7 +2132,7 @@ __global__ void __launch_bounds__(128, 8) k_lists(const __grid_constant__ Rebuil
             q = q2;
             left = left2;
             left2 = 0;
-            ox = wl ? o.x : o.x - bx;
+            ox = wl || fold ? o.x : o.x - (float)N.box[0];
         }
     }
     if (widest > longest) {
@@ -2877,10 +2884,10 @@ cudaError_t launch_rebuild(const RebuildArgs& R, int ntiles, int block, int nb, 
     } else if (nb > 0 && nb <= kGroupedBeads) {
         launch_lists_group<4>(R, nb, ncells, s);
     } else if (nb > 0) {
-        if (R.uniform == FN_CONST_ALL)
-            launch_next(k_lists<true>, (nb + 127) / 128, 128, 0, s, R, ncells);
-        else
-            launch_next(k_lists<false>, (nb + 127) / 128, 128, 0, s, R, ncells);
+        const bool all = R.uniform == FN_CONST_ALL;
+        launch_next(R.fold ? (all ? k_lists<true, true> : k_lists<false, true>)
+                           : (all ? k_lists<true, false> : k_lists<false, false>),
+                    (nb + 127) / 128, 128, 0, s, R, ncells);
     }
     /* the staged step kernel's copy, one block per tile (tiles are at most
        block - 4 beads wide) */

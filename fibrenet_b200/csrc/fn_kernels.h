@@ -242,6 +242,7 @@ struct RebuildArgs {
     int* csr;
     long long csr_region;
     int* tile_items;
+    int fold; /* some network folds its FP32 separations (list_fold) */
     int uniform; /* FN_CONST_* */
     FnNet net0;
     FnPair pair0;

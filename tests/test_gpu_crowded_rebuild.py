@@ -69,3 +69,15 @@ def rebuild_ms(m, build, cap):
 def test_capacity_of_long_rows_costs_no_time(n, side, build):
     m = gas(n, side, 1.8, seed=3)
     assert rebuild_ms(m, build, 26) < 1.4 * rebuild_ms(m, build, 256)
+
+
+# networks of three cells a side (folded separations) and of eight in one
+# context, below and above the size of the four-lane default
+@pytest.mark.parametrize("n", [2000, 101_000])
+def test_batch_of_short_and_long_boxes(n):
+    ms = [gas(600, 3, 1.2, seed=5), gas(n, round((n / 8) ** (1 / 3)), 1.2, seed=6), gas(800, 4, 1.2, mask=2, seed=7),
+          gas(n + 50, round((n / 6) ** (1 / 3)), 1.2, seed=8)]
+    want = lists(ms, "bricks", 16)
+    for build in ("beads", "groups"):
+        for a, b in zip(lists(ms, build, 16), want):
+            np.testing.assert_array_equal(a, b, err_msg=build)

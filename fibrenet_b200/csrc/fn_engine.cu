@@ -92,6 +92,11 @@ void set_list_radii(FnNet& N, const NetHost& h, double smax, double rmin, double
     N.list_in_r2 = out_ok && in_ok && !N.list_fold ? std::nextafter((float)(in * in * (1.0 - 1e-6)), 0.0f) : -1.0f;
 }
 
+/* A radius or skin radius as the least of its network takes it.  One that is
+   not a number is near no other, at whatever distance, so it counts as minus
+   infinity, which leaves its network without an inner radius. */
+double least(float v) { return std::isnan(v) ? -std::numeric_limits<double>::infinity() : (double)v; }
+
 /* the skin radius the upload gives a bead */
 double skin_of(double radius, double skin_ratio) { return (double)(float)(radius + skin_ratio); }
 
@@ -1272,7 +1277,7 @@ static int net_preamble(fn_ctx* c, int k, const fn_network_desc& d, long long& n
             const float rad = (float)d.radius[i];
             const float skin = (float)((double)rad + d.settings.skin_ratio);
             r = std::max(r, (double)rad);
-            lo = std::min(lo, (double)rad);
+            lo = std::min(lo, least(rad));
             sm = std::max(sm, (double)skin);
             g = std::min(g, (double)skin - (double)rad);
         }
@@ -2145,8 +2150,8 @@ FN_API int fn_set_skin(fn_ctx* c, const double* skin) {
         for (int i = c->info[k].bead_begin; i < c->info[k].bead_end; ++i) {
             smax = std::max(smax, (double)(float)skin[i]);
             gap = std::min(gap, (double)(float)skin[i] - (double)radius[i]);
-            rmin = std::min(rmin, (double)radius[i]);
-            smin = std::min(smin, (double)(float)skin[i]);
+            rmin = std::min(rmin, least(radius[i]));
+            smin = std::min(smin, least((float)skin[i]));
         }
         c->info[k].skin_gap = gap;
         set_list_radii(c->nets_h[k], c->info[k], smax, rmin, smin);

@@ -77,7 +77,8 @@ __global__ void __launch_bounds__(256) k_up_beads_check(const UpNet* __restrict_
         if (t < 0 || t >= N.n_types || !(mass >= 0.0)) atomicMin(&out[k].bad_bead, i);
         const float rad = (float)R.radius[u];
         const float skin = (float)((double)rad + N.skin_ratio);
-        kr = km = dkey((double)rad);
+        kr = dkey((double)rad);
+        km = rad == rad ? kr : dkey(-INFINITY); /* no inner listing radius */
         ks = dkey((double)skin);
         kg = dkey((double)skin - (double)rad);
     }

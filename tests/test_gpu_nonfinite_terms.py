@@ -33,3 +33,33 @@ def test_infinite_angle_stiffness(oracle_built, kw):
         assert np.isinf(o.get("force")).sum() > 8
         for f in ("force", "vel_old"):
             np.testing.assert_array_equal(s.get(f), o.get(f), err_msg=f)
+
+
+# a radius that is not a number is near no other: the list builds that test in
+# FP32 first against the build by bricks, which tests in FP64
+@pytest.mark.parametrize("value", [np.nan, np.inf, -np.inf])
+@pytest.mark.parametrize("later", [False, True])
+@pytest.mark.parametrize("host", [False, True])
+def test_lists_with_a_radius_or_skin_that_is_no_number(host, later, value):
+    from fibrenet_b200.native import Simulation
+    rng = np.random.default_rng(5)
+    st = Settings(dt=0.001, cutoff=1.0, box_unit_cell=2.0, box=(12.0, 14.0, 16.0), bc_type=0)
+    m = g.chain_model(rng.uniform(0.0, 12.0, (2000, 1, 3)), st, ["A"], [PAIR_HS], [[50.0, 0, 0, 0]], radius=0.5)
+    odd = np.arange(0, m.n_beads, 50)
+    skin = np.full(m.n_beads, 0.8)
+    if later:
+        skin[odd] = value
+    else:
+        m.radius[odd] = value
+    got = []
+    for build in ("bricks", "beads", "groups"):
+        with Simulation(m, list_capacity=256, host_upload=host) as s:
+            s.set_list_build(build)
+            if later:
+                s.set_skin(skin)
+            s.rebuild()
+            got.append(s.lists())
+    assert later is False or np.isinf(value) or got[0][0].sum() > 0
+    for c, p in got[1:]:
+        np.testing.assert_array_equal(c, got[0][0])
+        np.testing.assert_array_equal(p, got[0][1])
